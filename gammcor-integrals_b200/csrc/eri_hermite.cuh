@@ -18,14 +18,25 @@
 // contracted quartet, and the ket side carries only the columns a stage
 // keeps (pivot columns in the full-dimension stage, Step2.f90:242-419).
 //
-// Per primitive quartet the inner sum is a dense product
-//     X_i(h, J) += R~_ik(h, g) Ec_k(g, J),    R~(h, g) = R(h + g)
-// of H1 x H2 by H2 x nJ, and per row primitive pair O(r, J) += Er_i(r, h) X_i(h, J).
-// One warp evaluates one (row pair, column chunk) task: R_ik in warp-private
-// shared memory (level recursion, Helgaker 9.9.18-20), the Hankel operand
-// gathered from it through a per-block index table, the column vectors read
-// as ready-made B fragments, X and O in registers as DMMA accumulators; X is
-// turned into B fragments of the row product by warp shuffles.
+// Row primitive pairs are taken in blocks of IB and column primitive pairs in
+// groups of KP, so that the products have no padding between primitive pairs:
+//     X((i,h), J) += sum_{(k,g)} R_ik(h + g) Ec((k,g), J)
+// over the IB H1 rows of a block and the KP H2 columns of a group, then
+//     O(r, J) += sum_{(i,h)} Er(r, (i,h)) X((i,h), J)
+// per block.  One warp evaluates one (row pair, column chunk) task.
+//
+// The R_tuv of a batch of primitive quartets are evaluated one quartet per
+// lane (or per SL lanes), entirely in registers (hm_quartet), and left in
+// warp-private shared memory; the products then gather their Hankel operand from there through a
+// table of byte offsets, one 16-byte table load per eight fragments.  A unit is
+// one (block, group) combination of IB KP quartets; a batch holds UB of them.
+//
+// Bound by the FP64 tensor pipe where tasks are many (12 atoms of s4p3d2f1 with
+// 3-6 primitives, 4912 vectors: step-1 columns 1477 -> 830 ms, full-dimension
+// stage 1269 -> 648 ms against a form that took one primitive quartet at a time,
+// built its R level by level with 32 lanes in shared memory between the tensor
+// instructions, and padded every primitive pair to whole tiles).  Warps: 12 an SM
+// at 168 registers while the accumulators are few, else 8 with up to 255.
 #pragma once
 #include "gci_common.h"
 #include "boys.cuh"
@@ -37,29 +48,35 @@ template <int L1, int L2, int NT>
 struct HmShape {
     static constexpr int LT = L1 + L2;
     static constexpr int H1 = herm_n(L1), H2 = herm_n(L2), HT = herm_n(LT);
+    static constexpr int IB = hm_ib(L1), KP = hm_kp(L2), UQ = IB * KP;
     static constexpr int MT = hm_mt(L1), KT = hm_kt(L2), MTO = hm_mto(L1);
     static constexpr int RSTR = hm_row_stride(L1), CSTR = hm_col_stride(L2, NT);
-    static constexpr int KB = 32;          // column primitive pairs prepared at once (one per lane)
-    static constexpr int FS = LT + 4;      // per prepared primitive pair: F_0..F_LT, X, Y, Z
-    static constexpr int RS = HT + 1;      // R buffer, the last slot stays zero (padding of the gather)
+    static constexpr int TILES = MT * NT;
+    // 4 warps a block; 3 blocks an SM (168 registers a thread) while the accumulators are few
+    static constexpr int WARPS = 4, TPB = 32 * WARPS, MINB = TILES <= 12 ? 3 : 2;
+    // doubles of a quartet's R in the batch: odd, so that lanes storing the same entry of
+    // consecutive quartets fall into different banks
+    static constexpr int QS = HT | 1;
+    // ring of column fragments: PD k-steps, copied PD - 1 steps ahead
+    static constexpr int PD = TILES >= 8 ? 4 : 8;
+    static constexpr int RING = PD * NT * 32;
     static constexpr int OS = MTO * 8 * NT * 8;   // output block O(r, J), fragment order [MTO][NT][32][2]
-    static constexpr int WS = 3 * RS + KB * FS + OS;
-    // eight warps share the block's tables; (f,f|f,f) with three column tiles
-    // fills 226 KB of shared memory
-    static constexpr int WARPS = 8, TPB = 32 * WARPS;
-    // independent accumulator sets over alternating k-steps, so that at least
-    // ~12 tensor-core products are in flight per warp when the tile count is small
-    static constexpr int ACC0 = (12 + MT * NT - 1) / (MT * NT);
-    static constexpr int ACC = ACC0 > 4 ? 4 : ACC0;
-    // blocks per SM the launch bounds ask for: two when the accumulators are few
-    static constexpr int MINB = ACC * MT * NT * 2 <= 24 ? 2 : 1;
+    // table of byte offsets: [KT][32][MTP] 16-bit entries
+    static constexpr int MTP = MT <= 2 ? 2 : (MT <= 4 ? 4 : (MT + 3) / 4 * 4);
+    static constexpr int TAB = KT * 32 * MTP;   // shorts
+    // units of a batch: at most 32 quartets (one per lane) within the warp's share of 227 KB
+    static constexpr int BUDGET = ((MINB == 3 ? 74 : 112) * 1024 - 2 * TAB) / (8 * WARPS) - RING - OS;   // doubles
+    static constexpr int UB_MEM = BUDGET / (UQ * QS), UB_LANE = UQ >= 32 ? 1 : 32 / UQ;
+    static constexpr int UB = UB_MEM < 1 ? 1 : (UB_MEM < UB_LANE ? UB_MEM : UB_LANE);
+    static constexpr int RSZ = (UB * UQ * QS + 1) & ~1;
+    // lanes per quartet of the R recursion
+    static constexpr int SL = UB * UQ * 4 <= 32 && LT >= 4 ? 4 : (UB * UQ * 2 <= 32 && LT >= 2 ? 2 : 1);
+    static constexpr int WS = RSZ + RING + OS;
     // the next k-step's Hankel fragments are loaded one step ahead (registers: 2 MT)
     static constexpr bool APF = MT <= 7;
-    static constexpr size_t smem_bytes()
-    {
-        return sizeof(double) * ((size_t)WARPS * WS + HT) + sizeof(int) * (size_t)HT +
-               sizeof(short) * (size_t)MT * KT * 32;
-    }
+    static constexpr size_t smem_bytes() { return sizeof(double) * (size_t)WARPS * WS + sizeof(short) * (size_t)TAB; }
+    static_assert(UQ * QS * 8 <= 65535, "unit offsets are 16-bit");
+    static_assert(sizeof(double) * (size_t)WARPS * WS + 2 * TAB <= 227 * 1024, "shared memory");
 };
 
 template <int I, int N, class Fn>
@@ -80,67 +97,173 @@ __device__ __forceinline__ void dmma884(double (&d)[2], double a, double b)
         : "d"(a), "d"(b));
 }
 
-// One level of the Hermite Coulomb recursion (Helgaker 9.9.18-20):
-//   R^{(j)}_{tuv} = d R^{(j+1)}_{tuv - e} + (n - 1) R^{(j+1)}_{tuv - 2e}
-// along the first nonzero axis e of (t,u,v), with component n and d = X, Y or
-// Z, for every t+u+v <= LT - j, from `src` (level j+1) into `dst`; the
-// (0,0,0) entry takes F_j.  tab_rec packs the byte offsets of the two source
-// entries (bits 0-11, 12-23) and of d within fk[LT+1..LT+3] (bits 24-31).
-template <int LT>
-__device__ __forceinline__ void hm_level(int j, const double* __restrict__ fk, const double* src, double* dst,
-                                         const int* __restrict__ tab_rec, const double* __restrict__ tab_coef,
-                                         int lane)
+// One step of the Hermite Coulomb recursion along one axis (Helgaker 9.9.18-20)
+// for all orders n at fixed other components:
+//   R^{(n)}_{c} = d R^{(n+1)}_{c-1} + (c - 1) R^{(n+1)}_{c-2},  n = 0 .. M - c
+// from p1 = R_{c-1} (orders 0..M-c+1) and p2 = R_{c-2}; result over p2.
+template <int M, int C, int N1, int N2>
+__device__ __forceinline__ void hm_axis_step(double d, const double (&p1)[N1], double (&p2)[N2])
 {
-    const int nent = herm_n(LT - j);
-    const double Fj = fk[j];
-    const char* sb = reinterpret_cast<const char*>(src);
-    const char* db = reinterpret_cast<const char*>(fk + LT + 1);
-    for (int h = lane; h < nent; h += 32) {
-        const int rc = tab_rec[h];
-        const double d = *reinterpret_cast<const double*>(db + (rc >> 24));
-        const double r1 = *reinterpret_cast<const double*>(sb + (rc & 0xfff));
-        const double r2 = *reinterpret_cast<const double*>(sb + ((rc >> 12) & 0xfff));
-        const double r = fma(tab_coef[h], r2, d * r1);
-        dst[h] = h == 0 ? Fj : r;
-    }
+#pragma unroll
+    for (int n = 0; n <= M - C; ++n) p2[n] = C > 1 ? fma((double)(C - 1), p2[n + 1], d * p1[n + 1]) : d * p1[n + 1];
 }
+
+// R_tuv = R^{(0)}_tuv, t+u+v <= LT, of one primitive quartet from
+// F^{(n)} = (-2 alpha)^n pref F_n, stored at out[hm_ridx(LT,t,u,v)].  The levels
+// are walked axis by axis: the order-n row of R_{00v} gives the rows R_{0uv},
+// and those the R_{tuv}, so only two rows per axis are live (a level-by-level
+// recursion holds all herm_n(LT) values).  The same number of operations.
+// S lanes share a quartet when a batch holds fewer than 32: lane s takes the
+// planes v = S j + s, all lanes running the code of plane S j (its orders
+// beyond a lane's plane are not stored): 2.2 to 2.4 times fewer instructions
+// per quartet at S = 4.
+template <int LT, int S>
+__device__ __forceinline__ void hm_quartet(double (&F)[LT + 1], double X, double Y, double Z, int s,
+                                           double* __restrict__ out)
+{
+    double a0[LT + 1], a1[LT + 1];   // rows v - 1 (or v - 2 before the step) and v
+#pragma unroll
+    for (int n = 0; n <= LT; ++n) a1[n] = F[n];
+    hm_static_for<0, LT / S + 1>([&](auto J) {
+        constexpr int v0 = decltype(J)::value * S, MV = LT - v0;
+        double b0[MV + 1], b1[MV + 1];
+        hm_static_for<0, (S < MV + 1 ? S : MV + 1)>([&](auto W) {
+            constexpr int v = v0 + decltype(W)::value;
+            if constexpr (v == 1) {
+#pragma unroll
+                for (int n = 0; n <= LT; ++n) a0[n] = a1[n];
+                hm_axis_step<LT, 1>(Z, a0, a1);
+            } else if constexpr (v > 1) {
+                // a1 holds v - 1, a0 holds v - 2
+                hm_axis_step<LT, v>(Z, a1, a0);
+#pragma unroll
+                for (int n = 0; n <= LT; ++n) { const double t = a0[n]; a0[n] = a1[n]; a1[n] = t; }
+            }
+            if constexpr (v == v0) {
+#pragma unroll
+                for (int n = 0; n <= MV; ++n) b1[n] = a1[n];
+            } else {
+#pragma unroll
+                for (int n = 0; n <= LT - v; ++n) b1[n] = s == v - v0 ? a1[n] : b1[n];
+            }
+        });
+        const int vl = v0 + s;   // this lane's plane
+        double* __restrict__ pl = out + hm_ridx(LT, 0, 0, vl <= LT ? vl : LT);
+        hm_static_for<0, MV + 1>([&](auto U) {
+            constexpr int u = decltype(U)::value, MU = MV - u;
+            if constexpr (u == 1) {
+#pragma unroll
+                for (int n = 0; n <= MV; ++n) b0[n] = b1[n];
+                hm_axis_step<MV, 1>(Y, b0, b1);
+            } else if constexpr (u > 1) {
+                hm_axis_step<MV, u>(Y, b1, b0);
+#pragma unroll
+                for (int n = 0; n <= MV; ++n) { const double t = b0[n]; b0[n] = b1[n]; b1[n] = t; }
+            }
+            double c0[MU + 1], c1[MU + 1];
+#pragma unroll
+            for (int n = 0; n <= MU; ++n) c1[n] = b1[n];
+            hm_static_for<0, MU + 1>([&](auto T) {
+                constexpr int t = decltype(T)::value;
+                if constexpr (t == 1) {
+#pragma unroll
+                    for (int n = 0; n <= MU; ++n) c0[n] = c1[n];
+                    hm_axis_step<MU, 1>(X, c0, c1);
+                } else if constexpr (t > 1) {
+                    hm_axis_step<MU, t>(X, c1, c0);
+#pragma unroll
+                    for (int n = 0; n <= MU; ++n) { const double w = c0[n]; c0[n] = c1[n]; c1[n] = w; }
+                }
+                // planes v0 + s with LT - v0 - s < t + u do not have this entry
+                if (S == 1 || t + u <= MV - (S - 1) || s <= MV - t - u) pl[hm_ridx(LT, t, u, 0)] = c1[0];
+            });
+        });
+    });
+}
+
+// R of the primitive quartet (row primitive record Bp, column primitive record Kp),
+// all zero when !on (padding of a unit); s: this lane's share of the S.  One
+// function per level and split, called once per lane and batch.
+template <int LT, int S>
+__device__ __noinline__ void hm_produce(const double* __restrict__ Bp, const double* __restrict__ Kp, double kappa,
+                                        const double* __restrict__ boys, int on, int s, double* __restrict__ out)
+{
+    const double P = __ldg(Bp), Q = __ldg(Kp);
+    const double dx = __ldg(Bp + 1) - __ldg(Kp + 1), dy = __ldg(Bp + 2) - __ldg(Kp + 2), dz = __ldg(Bp + 3) - __ldg(Kp + 3);
+    // Boys values scaled by 2 pi^{5/2} / (PQ sqrt(P+Q+kappa PQ)) (auto2e_WMatrix_part1.f90:134)
+    // and (-2 alpha)^m
+    const double PQ = P * Q;
+    const double den = P + Q + kappa * PQ;
+    const double alpha = PQ / den;
+    const double pref = on ? 34.986836655249725 / (PQ * sqrt(den)) : 0.0;
+    double F[LT + 1];
+    boys_fm<LT>(alpha * (dx * dx + dy * dy + dz * dz), boys, F);
+    double pw = pref;
+    const double m2a = -2.0 * alpha;
+#pragma unroll
+    for (int m = 0; m <= LT; ++m) { F[m] *= pw; pw *= m2a; }
+    hm_quartet<LT, S>(F, dx, dy, dz, s, out);
+}
+
+// 8-byte asynchronous copy global -> shared
+__device__ __forceinline__ void hm_cp8(uint32_t dst, const double* src)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
+}
+
+// table words of one lane and k-step: MTP 16-bit byte offsets
+template <int MTP>
+struct HmIdx {
+    uint32_t w[MTP / 2];
+    __device__ __forceinline__ void load(const unsigned short* p)
+    {
+        if constexpr (MTP == 2) {
+            w[0] = *reinterpret_cast<const uint32_t*>(p);
+        } else if constexpr (MTP % 8 == 0) {
+#pragma unroll
+            for (int q = 0; q < MTP / 8; ++q) {
+                const uint4 v = reinterpret_cast<const uint4*>(p)[q];
+                w[4 * q] = v.x; w[4 * q + 1] = v.y; w[4 * q + 2] = v.z; w[4 * q + 3] = v.w;
+            }
+        } else {
+#pragma unroll
+            for (int q = 0; q < MTP / 4; ++q) {
+                const uint2 v = reinterpret_cast<const uint2*>(p)[q];
+                w[2 * q] = v.x; w[2 * q + 1] = v.y;
+            }
+        }
+    }
+    __device__ __forceinline__ uint32_t get(int m) const { return (m & 1) ? w[m >> 1] >> 16 : w[m >> 1] & 0xffffu; }
+};
 
 template <int L1, int L2, int NT>
 __global__ void __launch_bounds__(HmShape<L1, L2, NT>::TPB, HmShape<L1, L2, NT>::MINB)
 k_eri_hm(const HmArgs a)
 {
     using S = HmShape<L1, L2, NT>;
-    constexpr int LT = S::LT, HT = S::HT, MT = S::MT, KT = S::KT, MTO = S::MTO, ACC = S::ACC;
-    extern __shared__ double smem[];
-    double* tab_coef = smem + (size_t)S::WARPS * S::WS;
-    int* tab_rec = reinterpret_cast<int*>(tab_coef + HT);
-    short* tab_gidx = reinterpret_cast<short*>(tab_rec + HT);
+    constexpr int LT = S::LT, MT = S::MT, KT = S::KT, MTO = S::MTO, IB = S::IB, KP = S::KP, UQ = S::UQ, UB = S::UB;
+    constexpr int PD = S::PD;
+    extern __shared__ __align__(16) double smem[];
+    unsigned short* tab = reinterpret_cast<unsigned short*>(smem + (size_t)S::WARPS * S::WS);
 
-    for (int c = threadIdx.x; c < HT; c += S::TPB) {
-        const int t = herm_t(c), u = herm_u(c), v = herm_v(c);
-        int ax = 0, i1 = 0, i2 = 0, n = 0;
-        if (t > 0) { ax = 0; n = t; i1 = herm_idx(t - 1, u, v); i2 = t > 1 ? herm_idx(t - 2, u, v) : 0; }
-        else if (u > 0) { ax = 1; n = u; i1 = herm_idx(t, u - 1, v); i2 = u > 1 ? herm_idx(t, u - 2, v) : 0; }
-        else if (v > 0) { ax = 2; n = v; i1 = herm_idx(t, u, v - 1); i2 = v > 1 ? herm_idx(t, u, v - 2) : 0; }
-        tab_rec[c] = (8 * i1) | ((8 * i2) << 12) | ((8 * ax) << 24);
-        tab_coef[c] = n > 1 ? (double)(n - 1) : 0.0;
-    }
-    // A fragment (mt, ks) of the Hankel operand: lane l reads R(h + g) with
-    // h = 8 mt + l/4, g = 4 ks + l%4; padding reads the zero slot HT
-    for (int c = threadIdx.x; c < MT * KT * 32; c += S::TPB) {
-        const int l = c & 31, f = c >> 5;
-        const int mt = f / KT, ks = f - mt * KT;
-        const int h = 8 * mt + (l >> 2), g = 4 * ks + (l & 3);
-        int idx = HT;
-        if (h < S::H1 && g < S::H2)
-            idx = herm_idx(herm_t(h) + herm_t(g), herm_u(h) + herm_u(g), herm_v(h) + herm_v(g));
-        tab_gidx[c] = (short)idx;
+    // Hankel fragment (m, ks) of a unit: lane l reads R_{il,kl}(h + g) with (il, h) = 8 m + l/4 and
+    // (kl, g) = 4 ks + l%4 flattened over the unit's rows and columns.  Padding reads entry 0 (a
+    // finite value): its column vectors or its row vectors are zero.
+    for (int c = threadIdx.x; c < S::TAB; c += S::TPB) {
+        const int m = c % S::MTP, l = (c / S::MTP) & 31, ks = c / (S::MTP * 32);
+        const int rho = 8 * m + (l >> 2), kap = 4 * ks + (l & 3);
+        int off = 0;
+        if (rho < IB * S::H1 && kap < KP * S::H2) {
+            const int il = rho / S::H1, h = rho - il * S::H1, kl = kap / S::H2, g = kap - kl * S::H2;
+            off = 8 * ((il * KP + kl) * S::QS + hm_ridx(LT, herm_t(h) + herm_t(g), herm_u(h) + herm_u(g), herm_v(h) + herm_v(g)));
+        }
+        tab[c] = (unsigned short)off;
     }
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    double* Rb = smem + (size_t)warp * S::WS;   // three R buffers of RS doubles
-    double* Fk = Rb + 3 * S::RS;
-    double* Os = Fk + S::KB * S::FS;
-    if (lane < 3) Rb[lane * S::RS + HT] = 0.0;
+    double* Rb = smem + (size_t)warp * S::WS;
+    double* ring = Rb + S::RSZ + lane;
+    double* Os = Rb + S::RSZ + S::RING;
+    const uint32_t ring_s = (uint32_t)__cvta_generic_to_shared(ring);
     __syncthreads();
 
     const int64_t ntasks = a.nrows * a.nchunks;
@@ -157,11 +280,13 @@ k_eri_hm(const HmArgs a)
         const ShellPairDev pr = a.pairs[rp];
         const ShellPairDev pc = a.pairs[ch.pair];
         const int nb = pr.npp, nk = pc.npp;
+        const int nib = (nb + IB - 1) / IB, nkg = (nk + KP - 1) / KP, nu = nib * nkg;
         const int rsr = pp_record(pr.l1, pr.l2), rsc = pp_record(pc.l1, pc.l2);
         const double* __restrict__ rrec = a.pp + pr.rec_off;
         const double* __restrict__ crec = a.pp + pc.rec_off;
         const double* __restrict__ rowv = a.rowvec + a.rowvec_off[rp];
-        const double* __restrict__ colv = a.colvec + ch.vec_off;
+        const double* __restrict__ colv = a.colvec + ch.vec_off + lane;
+        const double* const colv_end = colv + (size_t)nkg * S::CSTR;
         const int first = pr.swap ? pr.s2 : pr.s1, second = pr.swap ? pr.s1 : pr.s2;
         const int n1 = __ldg(a.sh_nfunc + first);
         const int nR = n1 * __ldg(a.sh_nfunc + second);
@@ -169,158 +294,147 @@ k_eri_hm(const HmArgs a)
         // each lane owns entries 2 lane + {0,1} of every 64-entry tile of the block
         for (int w = 2 * lane; w < S::OS; w += 64) { Os[w] = 0.0; Os[w + 1] = 0.0; }
 
-        for (int i = 0; i < nb; ++i) {
-            const double* __restrict__ Bp = rrec + (size_t)i * rsr;
-            const double P = __ldg(Bp + 0), px = __ldg(Bp + 1), py = __ldg(Bp + 2), pz = __ldg(Bp + 3);
-            double X[ACC][MT][NT][2];
+        // the column fragments of all units in order, PD - 1 k-steps ahead (each lane copies and
+        // reads its own elements); every block of rows runs through the same column vectors
+        const double* cpf = colv;
+        uint32_t slot_w = 0, slot_r = 0;
+        auto prefetch = [&]() {
 #pragma unroll
-            for (int u = 0; u < ACC; ++u)
+            for (int n = 0; n < NT; ++n) hm_cp8(ring_s + 8 * (slot_w * NT + n) * 32, cpf + n * 32);
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            slot_w = (slot_w + 1) & (PD - 1);
+            cpf += NT * 32;
+            if (cpf == colv_end) cpf = colv;
+        };
+        if (nu > 0) {
+#pragma unroll
+            for (int s = 0; s < PD - 1; ++s) prefetch();
+        }
+
+        double X[MT][NT][2];
+#pragma unroll
+        for (int m = 0; m < MT; ++m)
+#pragma unroll
+            for (int n = 0; n < NT; ++n) X[m][n][0] = X[m][n][1] = 0.0;
+        int ib = 0, kg = 0;   // block and group of the unit whose products come next
+
+        for (int u0 = 0; u0 < nu; u0 += UB) {
+            const int un = nu - u0 < UB ? nu - u0 : UB;
+            __syncwarp();
+            // R of the batch, one quartet per SL lanes
+#pragma unroll 1
+            for (int q = lane / S::SL; q < un * UQ; q += 32 / S::SL) {
+                const int ul = q / UQ, rq = q - ul * UQ;
+                const int u = u0 + ul, uib = u / nkg, ukg = u - uib * nkg;
+                int i = uib * IB + rq / KP, k = ukg * KP + rq % KP;
+                const int on = i < nb && k < nk;
+                if (!on) i = k = 0;
+                hm_produce<LT, S::SL>(rrec + (size_t)i * rsr, crec + (size_t)k * rsc, a.kappa, a.boys, on,
+                                      lane % S::SL, Rb + q * S::QS);
+            }
+            __syncwarp();
+            const char* Ru = reinterpret_cast<const char*>(Rb);
+            for (int ul = 0; ul < un; ++ul) {
+                // rows of the block in use: whole tiles of its primitive pairs (blocks of one pair are full)
+                const int mte = (IB == 1 || (ib + 1) * IB <= nb) ? MT : ((nb - ib * IB) * S::H1 + 7) / 8;
+                const char* const Rn = ul + 1 < un ? Ru + UQ * S::QS * 8 : Ru;
+                auto steps = [&](auto FULL) {
+                    constexpr bool full = decltype(FULL)::value;
+                    const unsigned short* tp = tab + lane * S::MTP;
+                    double rn[S::APF ? MT : 1];
+                    if constexpr (S::APF) {
+                        HmIdx<S::MTP> ix;
+                        ix.load(tp);
+#pragma unroll
+                        for (int m = 0; m < MT; ++m) rn[m] = *reinterpret_cast<const double*>(Ru + ix.get(m));
+                    }
+#pragma unroll 1
+                    for (int ks = 0; ks < KT; ++ks) {
+                        asm volatile("cp.async.wait_group %0;" ::"n"(PD - 2) : "memory");
+                        double e[NT];
+#pragma unroll
+                        for (int n = 0; n < NT; ++n) e[n] = ring[(slot_r * NT + n) * 32];
+                        slot_r = (slot_r + 1) & (PD - 1);
+                        prefetch();
+                        if constexpr (S::APF) {
+                            double r[MT];
+#pragma unroll
+                            for (int m = 0; m < MT; ++m) r[m] = rn[m];
+                            tp += 32 * S::MTP;
+                            if (ks + 1 < KT) {
+                                HmIdx<S::MTP> ix;
+                                ix.load(tp);
+#pragma unroll
+                                for (int m = 0; m < MT; ++m) rn[m] = *reinterpret_cast<const double*>(Ru + ix.get(m));
+                            }
+#pragma unroll
+                            for (int m = 0; m < MT; ++m) {
+                                if (full || m < mte) {
+#pragma unroll
+                                    for (int n = 0; n < NT; ++n) dmma884(X[m][n], e[n], r[m]);
+                                }
+                            }
+                        } else {
+                            HmIdx<S::MTP> ix;
+                            ix.load(tp);
+                            tp += 32 * S::MTP;
+#pragma unroll
+                            for (int m = 0; m < MT; ++m) {
+                                const double r = *reinterpret_cast<const double*>(Ru + ix.get(m));
+#pragma unroll
+                                for (int n = 0; n < NT; ++n) dmma884(X[m][n], e[n], r);
+                            }
+                        }
+                    }
+                };
+                if (IB == 1 || mte == MT) steps(std::true_type{});
+                else steps(std::false_type{});
+                Ru = Rn;
+                if (++kg < nkg) continue;
+                // O(r, J) += Er(r, (i,h)) X((i,h), J): the accumulator element e of tile m holds row
+                // 8 m + 2 (l%4) + e of X at column J = l/4, which is a B fragment of k-step 2 m + e
+                // with the row vectors in that order
+                const double* __restrict__ rv = rowv + (size_t)ib * S::RSTR + lane;
+                constexpr int MO = NT >= 4 ? 1 : (NT >= 2 ? 2 : (MTO < 4 ? MTO : 4));   // output tiles at once
+#pragma unroll 1
+                for (int m0 = 0; m0 < MTO; m0 += MO) {
+                    if (8 * m0 >= nR) break;
+                    double acc[MO][NT][2];
+#pragma unroll
+                    for (int o = 0; o < MO; ++o)
+#pragma unroll
+                        for (int n = 0; n < NT; ++n) acc[o][n][0] = acc[o][n][1] = 0.0;
+#pragma unroll
+                    for (int ks = 0; ks < 2 * MT; ++ks)
+#pragma unroll
+                        for (int o = 0; o < MO; ++o) {
+                            if (MTO % MO != 0 && m0 + o >= MTO) continue;
+                            const double av = __ldg(rv + ((m0 + o) * 2 * MT + ks) * 32);
+#pragma unroll
+                            for (int n = 0; n < NT; ++n) dmma884(acc[o][n], av, X[ks >> 1][n][ks & 1]);
+                        }
+#pragma unroll
+                    for (int o = 0; o < MO; ++o) {
+                        if (MTO % MO != 0 && m0 + o >= MTO) continue;
+                        double2* od = reinterpret_cast<double2*>(Os + (m0 + o) * NT * 64 + 2 * lane);
+#pragma unroll
+                        for (int n = 0; n < NT; ++n) {
+                            double2 w = od[n * 32];
+                            w.x += acc[o][n][0];
+                            w.y += acc[o][n][1];
+                            od[n * 32] = w;
+                        }
+                    }
+                }
 #pragma unroll
                 for (int m = 0; m < MT; ++m)
 #pragma unroll
-                    for (int n = 0; n < NT; ++n) X[u][m][n][0] = X[u][m][n][1] = 0.0;
-
-            for (int k0 = 0; k0 < nk; k0 += S::KB) {
-                const int kn = (nk - k0) < S::KB ? (nk - k0) : S::KB;
-                for (int kk = lane; kk < kn; kk += 32) {
-                    // Boys values scaled by 2 pi^{5/2} / (PQ sqrt(P+Q+kappa PQ)) (auto2e_WMatrix_part1.f90:134)
-                    // and (-2 alpha)^m, and P - Q, of this row primitive with column primitive k0 + kk
-                    const double* __restrict__ Kp = crec + (size_t)(k0 + kk) * rsc;
-                    const double Q = __ldg(Kp + 0);
-                    const double dx = px - __ldg(Kp + 1), dy = py - __ldg(Kp + 2), dz = pz - __ldg(Kp + 3);
-                    const double PQ = P * Q;
-                    const double den = P + Q + a.kappa * PQ;
-                    const double alpha = PQ / den;
-                    const double pref = 34.986836655249725 / (PQ * sqrt(den));
-                    double F[LT + 1];
-                    boys_fm<LT>(alpha * (dx * dx + dy * dy + dz * dz), a.boys, F);
-                    double* fk = Fk + kk * S::FS;
-                    double pw = pref;
-                    const double m2a = -2.0 * alpha;
-#pragma unroll
-                    for (int m = 0; m <= LT; ++m) { fk[m] = F[m] * pw; pw *= m2a; }
-                    fk[LT + 1] = dx; fk[LT + 2] = dy; fk[LT + 3] = dz;
-                }
-                __syncwarp();
-                // R of the block's first primitive quartet; every later one is built
-                // level by level between the tensor-core steps of its predecessor
-                double* C = Rb;
-                double* src = Rb + S::RS;
-                double* dst = Rb + 2 * S::RS;
-                if (lane == 0) src[0] = Fk[LT];
-                __syncwarp();
-#pragma unroll 1
-                for (int j = LT - 1; j >= 0; --j) {
-                    hm_level<LT>(j, Fk, src, C, tab_rec, tab_coef, lane);
-                    __syncwarp();
-                    double* tmp = src; src = C; C = tmp;
-                }
-                { double* tmp = src; src = C; C = tmp; }   // C holds R^{(0)}
-                for (int kk = 0; kk < kn; ++kk) {
-                    const bool more = kk + 1 < kn;
-                    const double* fkn = Fk + (kk + 1) * S::FS;
-                    if (more && lane == 0) src[0] = fkn[LT];
-                    __syncwarp();
-                    // X(h, J) += R~(h, g) Ec(g, J), with the next quartet's recursion
-                    // levels spread over the k-steps
-                    const double* __restrict__ cv = colv + (size_t)(k0 + kk) * S::CSTR + lane;
-                    double bn[NT];
-#pragma unroll
-                    for (int n = 0; n < NT; ++n) bn[n] = __ldg(cv + n * 32);
-                    double an[S::APF ? MT : 1];
-                    if constexpr (S::APF) {
-#pragma unroll
-                        for (int m = 0; m < MT; ++m) an[m] = C[tab_gidx[m * KT * 32 + lane]];
-                    }
-                    int q = 0;
-#pragma unroll 1
-                    for (int ks0 = 0; ks0 < KT; ks0 += ACC) {
-                        hm_static_for<0, ACC>([&](auto U) {
-                            constexpr int u = decltype(U)::value;
-                            const int ks = ks0 + u;
-                            if (ks < KT) {
-                                double b[NT];
-#pragma unroll
-                                for (int n = 0; n < NT; ++n) b[n] = bn[n];
-                                if (ks + 1 < KT) {
-#pragma unroll
-                                    for (int n = 0; n < NT; ++n) bn[n] = __ldg(cv + ((ks + 1) * NT + n) * 32);
-                                }
-                                const short* gi = tab_gidx + ks * 32 + lane;
-                                if constexpr (S::APF) {
-                                    double av[MT];
-#pragma unroll
-                                    for (int m = 0; m < MT; ++m) av[m] = an[m];
-                                    if (ks + 1 < KT) {
-#pragma unroll
-                                        for (int m = 0; m < MT; ++m) an[m] = C[gi[m * KT * 32 + 32]];
-                                    }
-#pragma unroll
-                                    for (int m = 0; m < MT; ++m)
-#pragma unroll
-                                        for (int n = 0; n < NT; ++n) dmma884(X[u][m][n], av[m], b[n]);
-                                } else {
-#pragma unroll
-                                    for (int m = 0; m < MT; ++m) {
-                                        const double av = C[gi[m * KT * 32]];
-#pragma unroll
-                                        for (int n = 0; n < NT; ++n) dmma884(X[u][m][n], av, b[n]);
-                                    }
-                                }
-                                const int qe = more ? ((ks + 1) * LT) / KT : 0;
-                                for (; q < qe; ++q) {
-                                    hm_level<LT>(LT - 1 - q, fkn, src, dst, tab_rec, tab_coef, lane);
-                                    __syncwarp();
-                                    double* tmp = src; src = dst; dst = tmp;
-                                }
-                            }
-                        });
-                    }
-                    // the next quartet's R^{(0)} is in src; the free buffers rotate
-                    double* tmp = C; C = src; src = tmp;
-                    __syncwarp();
-                }
-            }
-            // O(r, J) += Er_i(r, h) X(h, J); the B fragment of k-step ks (h = 4 ks + l%4,
-            // J = 8 n + l/4) is held by lane 16 (ks%2) + 4 (l%4) + l/8 of X[ks/2][n]
-            if constexpr (ACC > 1) {
-#pragma unroll
-                for (int u = 1; u < ACC; ++u)
-#pragma unroll
-                    for (int m = 0; m < MT; ++m)
-#pragma unroll
-                        for (int n = 0; n < NT; ++n) { X[0][m][n][0] += X[u][m][n][0]; X[0][m][n][1] += X[u][m][n][1]; }
-            }
-            const double* __restrict__ rv = rowv + (size_t)i * S::RSTR + lane;
-            const int src0 = ((lane & 3) << 2) + (lane >> 3);
-            const bool odd = (lane >> 2) & 1;
-            // one 8-row tile of O at a time (even and odd k-steps in separate
-            // accumulators), added into the warp's block in shared memory
-#pragma unroll 1
-            for (int m = 0; m < MTO; ++m) {
-                if (8 * m >= nR) break;
-                double acc[2][NT][2];
-#pragma unroll
-                for (int n = 0; n < NT; ++n) acc[0][n][0] = acc[0][n][1] = acc[1][n][0] = acc[1][n][1] = 0.0;
-#pragma unroll
-                for (int ks = 0; ks < 2 * MT; ++ks) {
-                    const double av = __ldg(rv + (m * 2 * MT + ks) * 32);
-                    const int srcl = src0 + ((ks & 1) << 4);
-#pragma unroll
-                    for (int n = 0; n < NT; ++n) {
-                        const double v0 = __shfl_sync(0xffffffffu, X[0][ks >> 1][n][0], srcl);
-                        const double v1 = __shfl_sync(0xffffffffu, X[0][ks >> 1][n][1], srcl);
-                        dmma884(acc[ks & 1][n], av, odd ? v1 : v0);
-                    }
-                }
-                double* o = Os + (m * NT) * 64 + 2 * lane;
-#pragma unroll
-                for (int n = 0; n < NT; ++n) {
-                    o[n * 64] += acc[0][n][0] + acc[1][n][0];
-                    o[n * 64 + 1] += acc[0][n][1] + acc[1][n][1];
-                }
+                    for (int n = 0; n < NT; ++n) X[m][n][0] = X[m][n][1] = 0.0;
+                kg = 0;
+                ++ib;
             }
         }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
 
         // scatter: element (m, n, l, e) of the block is O(8 m + l/4, 8 n + 2 (l%4) + e)
 #pragma unroll 1

@@ -56,8 +56,9 @@ __device__ __forceinline__ void hm_canon(const ShellPairDev& d, const int* __res
     f2 = d.swap ? fa : fb;
 }
 
-// Row vectors of the listed pairs: per primitive pair [MTO][2 MT][32], element
-// (m, ks, l) = Er(r = 8 m + l/4, h = 4 ks + l%4); one block per pair.
+// Row vectors of the listed pairs: per block of primitive pairs [MTO][2 MT][32], element
+// (m, 2 j + e, l) = Er(r = 8 m + l/4, (i,h) = 8 j + 2 (l%4) + e) -- the k order in which the
+// accumulators of the first product are the B fragments of the second; one block per pair.
 __global__ void k_hm_rowvec(const int* __restrict__ ids, int nids, const ShellPairDev* __restrict__ pairs,
                             const double* __restrict__ pp, const int64_t* __restrict__ off,
                             const double* __restrict__ tmat, const int* __restrict__ toff,
@@ -67,19 +68,20 @@ __global__ void k_hm_rowvec(const int* __restrict__ ids, int nids, const ShellPa
         const int id = ids[q];
         const ShellPairDev d = pairs[id];
         const int L = d.l1 + d.l2;
-        const int H = herm_n(L), MT2 = 2 * hm_mt(L), stride = hm_row_stride(L);
+        const int H = herm_n(L), MT2 = 2 * hm_mt(L), stride = hm_row_stride(L), IB = hm_ib(L);
         const int nR = __ldg(nfunc + d.s1) * __ldg(nfunc + d.s2);
         const int rs = pp_record(d.l1, d.l2);
         double* __restrict__ out = vec + off[id];
-        const int64_t n = (int64_t)d.npp * stride;
+        const int64_t n = (int64_t)hm_row_blocks(L, d.npp) * stride;
         for (int64_t e = threadIdx.x; e < n; e += blockDim.x) {
-            const int i = (int)(e / stride);
-            const int w = (int)(e - (int64_t)i * stride);
+            const int ib = (int)(e / stride);
+            const int w = (int)(e - (int64_t)ib * stride);
             const int l = w & 31, f = w >> 5;
             const int m = f / MT2, ks = f - m * MT2;
-            const int r = 8 * m + (l >> 2), h = 4 * ks + (l & 3);
+            const int r = 8 * m + (l >> 2), rho = 8 * (ks >> 1) + 2 * (l & 3) + (ks & 1);
+            const int il = rho / H, h = rho - il * H, i = ib * IB + il;
             double val = 0.0;
-            if (r < nR && h < H) {
+            if (r < nR && il < IB && i < d.npp) {
                 int f1, f2;
                 hm_canon(d, nfunc, r, f1, f2);
                 val = hm_element(d, pp + d.rec_off + (size_t)i * rs, f1, f2, herm_t(h), herm_u(h), herm_v(h), tmat,
@@ -90,8 +92,8 @@ __global__ void k_hm_rowvec(const int* __restrict__ ids, int nids, const ShellPa
     }
 }
 
-// Column vectors of the chunks: per primitive pair [KT][NT][32], element
-// (ks, n, l) = (-1)^|g| Ec(g = 4 ks + l%4, J = 8 n + l/4); one block per chunk.
+// Column vectors of the chunks: per group of primitive pairs [KT][NT][32], element
+// (ks, n, l) = (-1)^|g| Ec((k,g) = 4 ks + l%4, J = 8 n + l/4); one block per chunk.
 __global__ void k_hm_colvec(const HmChunk* __restrict__ chunks, int nchunks, const ShellPairDev* __restrict__ pairs,
                             const double* __restrict__ pp, const int* __restrict__ colfun,
                             const double* __restrict__ tmat, const int* __restrict__ toff,
@@ -101,18 +103,19 @@ __global__ void k_hm_colvec(const HmChunk* __restrict__ chunks, int nchunks, con
         const HmChunk ch = chunks[q];
         const ShellPairDev d = pairs[ch.pair];
         const int L = d.l1 + d.l2;
-        const int H = herm_n(L), stride = hm_col_stride(L, ch.nt);
+        const int H = herm_n(L), stride = hm_col_stride(L, ch.nt), KP = hm_kp(L);
         const int rs = pp_record(d.l1, d.l2);
         double* __restrict__ out = vec + ch.vec_off;
-        const int64_t n = (int64_t)d.npp * stride;
+        const int64_t n = (int64_t)hm_col_groups(L, d.npp) * stride;
         for (int64_t e = threadIdx.x; e < n; e += blockDim.x) {
-            const int k = (int)(e / stride);
-            const int w = (int)(e - (int64_t)k * stride);
+            const int kg = (int)(e / stride);
+            const int w = (int)(e - (int64_t)kg * stride);
             const int l = w & 31, f = w >> 5;
             const int ks = f / ch.nt, nn = f - ks * ch.nt;
-            const int g = 4 * ks + (l & 3), J = 8 * nn + (l >> 2);
+            const int kap = 4 * ks + (l & 3), J = 8 * nn + (l >> 2);
+            const int kl = kap / H, g = kap - kl * H, k = kg * KP + kl;
             double val = 0.0;
-            if (g < H && J < ch.ncol) {
+            if (kl < KP && k < d.npp && J < ch.ncol) {
                 int f1, f2;
                 hm_canon(d, nfunc, colfun[ch.col_off + J], f1, f2);
                 const int t = herm_t(g), u = herm_u(g), v = herm_v(g);

@@ -541,7 +541,8 @@ static void hm_ensure_rows(Handle& H, const std::vector<int>& ids)
         if (!want[id]) continue;
         list.push_back((int)id);
         off[id] = tot;
-        tot += (int64_t)P.h[id].npp * hm_row_stride(P.h[id].l1 + P.h[id].l2);
+        const int L = P.h[id].l1 + P.h[id].l2;
+        tot += (int64_t)hm_row_blocks(L, P.h[id].npp) * hm_row_stride(L);
     }
     H.hm_rowvec.alloc((size_t)std::max<int64_t>(tot, 1));
     H.hm_rowoff.upload(off, C.stream);
@@ -596,7 +597,7 @@ static void run_eri_hm(Handle& H, const std::vector<int>& gb, const std::vector<
                     ch.nt = (cnt + 7) / 8;
                     ch.vec_off = voff;
                     ch.col_off = (int64_t)colfun.size();
-                    voff += (int64_t)d.npp * hm_col_stride(L, ch.nt);
+                    voff += (int64_t)hm_col_groups(L, d.npp) * hm_col_stride(L, ch.nt);
                     for (int j = beg; j < beg + cnt; ++j) { colfun.push_back(fl[j]); colout.push_back(ol[j]); }
                     beg += cnt;
                     group[gidx(w, tk, ch.nt)].push_back((int)chunks.size());
@@ -666,11 +667,13 @@ static void run_eri_hm(Handle& H, const std::vector<int>& gb, const std::vector<
         const int64_t nb = sb[tb + 1] - sb[tb];
         if (nb == 0) continue;
         const int L1 = type_lsum(tb);
-        double npb = 0.0, rowt = 0.0;
+        // 8-row tiles of the blocks, and k-steps x 8-row tiles of the row products
+        double rowm = 0.0, rowt = 0.0;
         for (int64_t q = sb[tb]; q < sb[tb + 1]; ++q) {
-            const int id = gb[q];
-            npb += P.h[id].npp;
-            rowt += (double)P.h[id].npp * ((P.nab[id] + 7) / 8);
+            const int id = gb[q], nib = hm_row_blocks(L1, P.h[id].npp);
+            if (nib == 0) continue;
+            rowm += (double)(nib - 1) * hm_mt(L1) + ((P.h[id].npp - (nib - 1) * hm_ib(L1)) * herm_n(L1) + 7) / 8;
+            rowt += (double)nib * 2.0 * hm_mt(L1) * ((P.nab[id] + 7) / 8);
         }
         const int w = hm_max_nt(L1);
         for (int tk = 0; tk < kNumPairTypes; ++tk)
@@ -679,9 +682,10 @@ static void run_eri_hm(Handle& H, const std::vector<int>& gb, const std::vector<
                 const int64_t nc = gstart[g + 1] - gstart[g];
                 if (nc == 0) continue;
                 const int L2 = type_lsum(tk);
-                double npk = 0.0;
-                for (int64_t q = gstart[g]; q < gstart[g + 1]; ++q) npk += P.h[chunks[order[q]].pair].npp;
-                const double fl = 512.0 * nt * (npb * npk * hm_mt(L1) * hm_kt(L2) + rowt * nc * 2.0 * hm_mt(L1));
+                double colk = 0.0;
+                for (int64_t q = gstart[g]; q < gstart[g + 1]; ++q)
+                    colk += (double)hm_col_groups(L2, P.h[chunks[order[q]].pair].npp) * hm_kt(L2);
+                const double fl = 512.0 * nt * (rowm * colk + rowt * nc);
                 H.hm_flops += fl;
                 double* cs = H.hm_class[L1][L2][nt - 1];
                 cs[0] += 1.0;

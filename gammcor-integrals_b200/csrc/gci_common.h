@@ -156,31 +156,45 @@ GCI_HD constexpr int hm_max_nf(int L)
     }
     return m;
 }
-GCI_HD constexpr int hm_mt(int L) { return (herm_n(L) + 7) / 8; }    // 8-row tiles over a Hermite index
-GCI_HD constexpr int hm_kt(int L) { return (herm_n(L) + 3) / 4; }    // 4-wide k-steps over a Hermite index
+// Row primitive pairs of one block: the block's ib herm_n(L1) rows fill whole 8-row tiles
+// (16, 32, 40, 40 rows for L1 = 0..3; 35, 56 and 84 rows in 5, 7 and 11 tiles above).
+GCI_HD constexpr int hm_ib(int L) { return L == 0 ? 16 : (L == 1 ? 8 : (L == 2 ? 4 : (L == 3 ? 2 : 1))); }
+// Column primitive pairs of one group: the group's kp herm_n(L2) columns fill whole 4-wide k-steps
+// (4, 4, 20, 20 columns for L2 = 0..3, 35, 56 and 84 above).
+GCI_HD constexpr int hm_kp(int L) { return L == 0 ? 4 : (L == 2 ? 2 : 1); }
+GCI_HD constexpr int hm_mt(int L) { return (hm_ib(L) * herm_n(L) + 7) / 8; }    // 8-row tiles of a block
+GCI_HD constexpr int hm_kt(int L) { return (hm_kp(L) * herm_n(L) + 3) / 4; }    // k-steps of a group
 GCI_HD constexpr int hm_mto(int L) { return (hm_max_nf(L) + 7) / 8; } // 8-row tiles over the row functions
-// doubles of one row primitive pair's vectors: [MTO][2 MT][32] (A fragments of the row product)
+// doubles of one block's row vectors: [MTO][2 MT][32] (A fragments of the row product)
 GCI_HD constexpr int hm_row_stride(int L) { return hm_mto(L) * 2 * hm_mt(L) * 32; }
-// doubles of one column primitive pair's vectors in a chunk of NT column tiles: [KT][NT][32]
+// doubles of one group's column vectors in a chunk of NT column tiles: [KT][NT][32]
 GCI_HD constexpr int hm_col_stride(int L, int nt) { return hm_kt(L) * nt * 32; }
+GCI_HD constexpr int hm_row_blocks(int L, int npp) { return (npp + hm_ib(L) - 1) / hm_ib(L); }
+GCI_HD constexpr int hm_col_groups(int L, int npp) { return (npp + hm_kp(L) - 1) / hm_kp(L); }
+// Position of R_tuv among the herm_n(LT) of a quartet: planes of constant v, within a plane by
+// t + u, then u.
+GCI_HD constexpr int hm_ridx(int LT, int t, int u, int v)
+{
+    return herm_n(LT) - herm_n(LT - v) + (t + u) * (t + u + 1) / 2 + u;
+}
 constexpr int kHmMaxNT = 7;   // column tiles per task, at most (56 columns)
 // Column tiles per task for rows of Hermite level L1: the 8x8 accumulator tiles of
-// X (ceil(H1/8) x NT) stay at about 30 or fewer (two doubles per lane each).
-GCI_HD constexpr int hm_max_nt(int L1) { return L1 <= 3 ? 7 : (L1 == 4 ? 5 : (L1 == 5 ? 4 : 3)); }
+// X (hm_mt x NT) stay at about 30 or fewer (two doubles per lane each).
+GCI_HD constexpr int hm_max_nt(int L1) { return L1 <= 1 ? 7 : (L1 <= 4 ? 5 : (L1 == 5 ? 4 : 3)); }
 
 // A group of at most 8 * NT requested columns of one column pair.
 struct HmChunk {
     int pair;          // pair id (all-pair index)
     int ncol;          // columns in the chunk
     int nt;            // column tiles of its vectors (ncol <= 8 nt)
-    int64_t vec_off;   // offset (doubles) of the chunk's vectors in colvec: [k][KT][NT][32]
+    int64_t vec_off;   // offset (doubles) of the chunk's vectors in colvec: [group][KT][NT][32]
     int64_t col_off;   // offset of the chunk's entries in colfun / colout
 };
 
 struct HmArgs {
     const ShellPairDev* pairs;
     const double* pp;            // primitive-pair records (P and the product centre at [0..3])
-    const double* rowvec;        // row vectors, per pair: [i][MTO][2 MT][32]
+    const double* rowvec;        // row vectors, per pair: [block][MTO][2 MT][32]
     const int64_t* rowvec_off;   // per pair id
     const HmChunk* chunks;
     const double* colvec;

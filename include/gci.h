@@ -238,7 +238,7 @@ int gci_eri_hm(int enable);
 
 /* Work of the Hermite-matrix kernels of a decomposition (and its gci_rkab
  * calls): for every row level L1 (0..6), column level L2 (0..6) and column
- * tile count (1..7, at most 7 for L1 <= 3, 5 for L1 = 4, 4 for L1 = 5, 3 for L1 = 6), in that
+ * tile count (1..7, at most 7 for L1 <= 1, 5 for L1 <= 4, 4 for L1 = 5, 3 for L1 = 6), in that
  * order: launches, device seconds (measured only with gci_eri_hm(2)) and
  * tensor-core flops issued (padding included); 7 x 7 x 7 x 3 values. */
 int gci_eri_hm_stats(const gci_handle *h, double *out, int n);

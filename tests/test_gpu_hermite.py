@@ -1,0 +1,38 @@
+"""GPU tests of the Hermite-matrix ERI kernels at the edges of their blocking:
+primitive-pair counts below, at and above the row blocks (16, 8, 4, 2 and 1
+primitive pairs) and column groups (4, 2, 1) of every Hermite level.
+
+Reference: the class kernels (gci_eri_hm(0)), an independent evaluation.
+Tolerance: both sum the same FP64 products of each integral, at most a few
+thousand terms no larger than the largest integral's, in different orders:
+1e-12 of the largest integral (the bound of the ERI parity tests).
+"""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from gammcor_integrals_b200 import _capi, basis as gbasis, molecules
+
+pytestmark = pytest.mark.gpu
+
+
+def _eri_pairs(lib, tb, omega, hm):
+    npq = tb.NAO * (tb.NAO + 1) // 2
+    out = np.full((npq, npq), np.nan, order="F")
+    s = tb.c_struct()
+    before = lib.gci_eri_hm(1 if hm else 0)
+    try:
+        _capi.check(lib.gci_eri_pairs(C.byref(s), omega, _capi.ptr(out), npq))
+    finally:
+        lib.gci_eri_hm(before)
+    return out
+
+
+@pytest.mark.parametrize("nprim,omega", [((1, 1), 0.0), ((2, 2), 0.0), ((1, 3), 0.5), ((3, 5), 0.0), ((6, 7), 0.0)])
+def test_blocks_and_groups_match_class_kernels(gpu_lib, nprim, omega):
+    # 1, 4, 1..9, 9..25 and 36..49 primitive pairs a shell pair before the screen
+    mol = molecules.random_molecule(31, 2, 4.0, (0, 1, 2, 3), nprim, (0.1, 50.0))
+    tb = gbasis.from_molecule(mol)
+    got, ref = _eri_pairs(gpu_lib, tb, omega, True), _eri_pairs(gpu_lib, tb, omega, False)
+    assert np.max(np.abs(got - ref)) <= 1e-12 * np.max(np.abs(ref))
