@@ -15,35 +15,70 @@
 
 namespace gci {
 
-// Coefficient of Hermite index (t,u,v) of the function pair (f1, f2) of the
-// canonical shells (s1, s2) of a pair in primitive-pair record `rec`.
-__device__ static double hm_element(const ShellPairDev& d, const double* __restrict__ rec, int f1, int f2, int t,
-                                    int u, int v, const double* __restrict__ tmat, const int* __restrict__ toff)
+// Index tables of a pair in shared memory: the powers of the Cartesian
+// components and of the Hermite indices, and the nonzero entries of the two
+// shells' transforms (one to three of the ncart(l) for most solid harmonics).
+// Elements are cheap sums over these lists, bound by the latency of their table
+// loads; decoding the indices and scanning the dense transforms for every
+// element cost several times the arithmetic (ERI matrix of 60 AOs with f shells
+// 63 -> 40 ms, the AO->MO transform at 210 AOs 237 -> 211 ms).
+struct HmPairTab {
+    int herm[herm_n(kMaxPairL)];              // t | u << 8 | v << 16
+    int nz[2][2 * kMaxL + 1];                 // nonzero entries of each function
+    int pw[2][2 * kMaxL + 1][ncart(kMaxL)];   // their powers x | y << 8 | z << 16
+    double w[2][2 * kMaxL + 1][ncart(kMaxL)]; // and weights, in the order of the components
+};
+
+// Fills the table for the pair d (all threads of the block; synchronises).
+__device__ static void hm_pair_tab(HmPairTab& T, const ShellPairDev& d, const double* __restrict__ tmat,
+                                   const int* __restrict__ toff, const int* __restrict__ nfunc)
 {
-    const int la = d.l1, lb = d.l2;
-    const int n1 = ncart(la), n2 = ncart(lb);
-    const int ne = e2_size(la, lb);
-    const double* __restrict__ Ex = rec + 8;
-    const double* __restrict__ Ey = Ex + ne;
-    const double* __restrict__ Ez = Ey + ne;
-    const double* __restrict__ T1 = tmat + __ldg(toff + d.s1) + f1 * n1;
-    const double* __restrict__ T2 = tmat + __ldg(toff + d.s2) + f2 * n2;
+    __syncthreads();   // the previous pair's readers are done
+    const int H = herm_n(d.l1 + d.l2);
+    for (int h = threadIdx.x; h < H; h += blockDim.x) T.herm[h] = herm_t(h) | (herm_u(h) << 8) | (herm_v(h) << 16);
+    if (threadIdx.x < 2 * (2 * kMaxL + 1)) {
+        const int which = threadIdx.x / (2 * kMaxL + 1), f = threadIdx.x % (2 * kMaxL + 1);
+        const int s = which ? d.s2 : d.s1, l = which ? d.l2 : d.l1, nc = ncart(l);
+        int n = 0;
+        if (f < __ldg(nfunc + s)) {
+            const double* __restrict__ t = tmat + __ldg(toff + s) + f * nc;
+            for (int c = 0; c < nc; ++c) {
+                const double w = __ldg(t + c);
+                if (w == 0.0) continue;
+                const int g = cart_off(l) + c;
+                T.pw[which][f][n] = cart_x(g) | (cart_y(g) << 8) | (cart_z(g) << 16);
+                T.w[which][f][n] = w;
+                ++n;
+            }
+        }
+        T.nz[which][f] = n;
+    }
+    __syncthreads();
+}
+
+// Coefficient of Hermite index (t,u,v) (packed) of the function pair (f1, f2) of the
+// canonical shells (s1, s2) of a pair in primitive-pair record `rec`.
+__device__ static double hm_element(const HmPairTab& T, const ShellPairDev& d, const double* __restrict__ rec, int f1,
+                                    int f2, int tuv)
+{
+    const int la = d.l1, ne = e2_size(la, d.l2);
+    const int t = tuv & 255, u = (tuv >> 8) & 255, v = tuv >> 16;
+    const double* __restrict__ Ex = rec + 8 + t;
+    const double* __restrict__ Ey = rec + 8 + ne + u;
+    const double* __restrict__ Ez = rec + 8 + 2 * ne + v;
     double sum = 0.0;
-    for (int c1 = 0; c1 < n1; ++c1) {
-        const double w1 = __ldg(T1 + c1);
-        if (w1 == 0.0) continue;
-        const int g1 = cart_off(la) + c1;
-        const int x1 = cart_x(g1), y1 = cart_y(g1), z1 = cart_z(g1);
-        for (int c2 = 0; c2 < n2; ++c2) {
-            const double w2 = __ldg(T2 + c2);
-            if (w2 == 0.0) continue;
-            const int g2 = cart_off(lb) + c2;
-            const int x2 = cart_x(g2), y2 = cart_y(g2), z2 = cart_z(g2);
+    for (int c1 = 0; c1 < T.nz[0][f1]; ++c1) {
+        const double w1 = T.w[0][f1][c1];
+        const int p1 = T.pw[0][f1][c1], x1 = p1 & 255, y1 = (p1 >> 8) & 255, z1 = p1 >> 16;
+        for (int c2 = 0; c2 < T.nz[1][f2]; ++c2) {
+            const double w2 = T.w[1][f2][c2];
+            const int p2 = T.pw[1][f2][c2], x2 = p2 & 255, y2 = (p2 >> 8) & 255, z2 = p2 >> 16;
             if (t > x1 + x2 || u > y1 + y2 || v > z1 + z2) continue;
-            sum += w1 * w2 * Ex[e2_off(la, x1, x2) + t] * Ey[e2_off(la, y1, y2) + u] * Ez[e2_off(la, z1, z2) + v];
+            sum += w1 * w2 * __ldg(Ex + e2_off(la, x1, x2)) * __ldg(Ey + e2_off(la, y1, y2)) *
+                   __ldg(Ez + e2_off(la, z1, z2));
         }
     }
-    return sum * rec[4];
+    return sum * __ldg(rec + 4);
 }
 
 // Stored-orientation function code f = f_first + N_first f_second -> canonical (f1, f2).
@@ -64,6 +99,7 @@ __global__ void k_hm_rowvec(const int* __restrict__ ids, int nids, const ShellPa
                             const double* __restrict__ tmat, const int* __restrict__ toff,
                             const int* __restrict__ nfunc, double* __restrict__ vec)
 {
+    __shared__ HmPairTab T;
     for (int q = blockIdx.x; q < nids; q += gridDim.x) {
         const int id = ids[q];
         const ShellPairDev d = pairs[id];
@@ -71,6 +107,7 @@ __global__ void k_hm_rowvec(const int* __restrict__ ids, int nids, const ShellPa
         const int H = herm_n(L), MT2 = 2 * hm_mt(L), stride = hm_row_stride(L), IB = hm_ib(L);
         const int nR = __ldg(nfunc + d.s1) * __ldg(nfunc + d.s2);
         const int rs = pp_record(d.l1, d.l2);
+        hm_pair_tab(T, d, tmat, toff, nfunc);
         double* __restrict__ out = vec + off[id];
         const int64_t n = (int64_t)hm_row_blocks(L, d.npp) * stride;
         for (int64_t e = threadIdx.x; e < n; e += blockDim.x) {
@@ -84,8 +121,7 @@ __global__ void k_hm_rowvec(const int* __restrict__ ids, int nids, const ShellPa
             if (r < nR && il < IB && i < d.npp) {
                 int f1, f2;
                 hm_canon(d, nfunc, r, f1, f2);
-                val = hm_element(d, pp + d.rec_off + (size_t)i * rs, f1, f2, herm_t(h), herm_u(h), herm_v(h), tmat,
-                                 toff);
+                val = hm_element(T, d, pp + d.rec_off + (size_t)i * rs, f1, f2, T.herm[h]);
             }
             out[e] = val;
         }
@@ -99,12 +135,14 @@ __global__ void k_hm_colvec(const HmChunk* __restrict__ chunks, int nchunks, con
                             const double* __restrict__ tmat, const int* __restrict__ toff,
                             const int* __restrict__ nfunc, double* __restrict__ vec)
 {
+    __shared__ HmPairTab T;
     for (int q = blockIdx.x; q < nchunks; q += gridDim.x) {
         const HmChunk ch = chunks[q];
         const ShellPairDev d = pairs[ch.pair];
         const int L = d.l1 + d.l2;
         const int H = herm_n(L), stride = hm_col_stride(L, ch.nt), KP = hm_kp(L);
         const int rs = pp_record(d.l1, d.l2);
+        hm_pair_tab(T, d, tmat, toff, nfunc);
         double* __restrict__ out = vec + ch.vec_off;
         const int64_t n = (int64_t)hm_col_groups(L, d.npp) * stride;
         for (int64_t e = threadIdx.x; e < n; e += blockDim.x) {
@@ -118,9 +156,9 @@ __global__ void k_hm_colvec(const HmChunk* __restrict__ chunks, int nchunks, con
             if (kl < KP && k < d.npp && J < ch.ncol) {
                 int f1, f2;
                 hm_canon(d, nfunc, colfun[ch.col_off + J], f1, f2);
-                const int t = herm_t(g), u = herm_u(g), v = herm_v(g);
-                val = hm_element(d, pp + d.rec_off + (size_t)k * rs, f1, f2, t, u, v, tmat, toff);
-                if ((t + u + v) & 1) val = -val;
+                const int tuv = T.herm[g];
+                val = hm_element(T, d, pp + d.rec_off + (size_t)k * rs, f1, f2, tuv);
+                if ((tuv ^ (tuv >> 8) ^ (tuv >> 16)) & 1) val = -val;
             }
             out[e] = val;
         }
