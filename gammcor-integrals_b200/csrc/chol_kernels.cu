@@ -3,6 +3,7 @@
 // diagonal and the reshaping kernels of the AO->MO transformation.
 #include "gci_common.h"
 #include "gci_runtime.h"
+#include <algorithm>
 #include <cfloat>
 
 namespace gci {
@@ -47,78 +48,139 @@ __device__ __forceinline__ bool better(double v, int i, double bv, int bi)
     return v > bv || (v == bv && i < bi);
 }
 
-// Block-wide argmax with the reference's tie rule: strict '>' scanning in
-// increasing index order, i.e. the largest value at the smallest index
-// (chol2_BatchMax, TwoStepCholesky_Step1.f90:720-727).
-__device__ void block_argmax(const double* __restrict__ v, int n, double& bestv, int& besti,
-                             double* s_v, int* s_i)
-{
-    double bv = -DBL_MAX;
-    int bi = 0x7fffffff;
-    for (int i = threadIdx.x; i < n; i += blockDim.x)
-        if (better(v[i], i, bv, bi)) { bv = v[i]; bi = i; }
-    for (int off = 16; off > 0; off >>= 1) {
-        const double ov = __shfl_down_sync(0xffffffffu, bv, off);
-        const int oi = __shfl_down_sync(0xffffffffu, bi, off);
-        if (better(ov, oi, bv, bi)) { bv = ov; bi = oi; }
-    }
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (lane == 0) { s_v[warp] = bv; s_i[warp] = bi; }
-    __syncthreads();
-    if (warp == 0) {
-        const int nw = (blockDim.x + 31) >> 5;
-        bv = lane < nw ? s_v[lane] : -DBL_MAX;
-        bi = lane < nw ? s_i[lane] : 0x7fffffff;
-        for (int off = 16; off > 0; off >>= 1) {
-            const double ov = __shfl_down_sync(0xffffffffu, bv, off);
-            const int oi = __shfl_down_sync(0xffffffffu, bi, off);
-            if (better(ov, oi, bv, bi)) { bv = ov; bi = oi; }
-        }
-        if (lane == 0) { s_v[0] = bv; s_i[0] = bi; }
-    }
-    __syncthreads();
-    bestv = s_v[0];
-    besti = s_i[0];
-    __syncthreads();
-}
-
 // Micro-iterations of one macro iteration (chol2_Pivots, Step1.f90:1025-1064)
 // restricted to the batch: the pivot choice depends only on the batch rows
-// of M and of the new vectors, so the sequential part runs in one CTA on the
-// nb x nb block Mbb; the vectors over all candidates follow afterwards as one
+// of M and of the new vectors, so the sequential part runs on the nb x nb
+// block Mbb; the vectors over all candidates follow afterwards as one
 // triangular solve.  Lb(:, j) = (Mbb(:, piv_j) - Lb Lb(piv_j, :)^T) / sqrt(Dmax_j).
-__global__ void __launch_bounds__(1024) k_pivot_batch(const double* __restrict__ Mbb, int nb, double* __restrict__ Db,
-                                                      double* __restrict__ Lb, int* __restrict__ piv,
-                                                      double* __restrict__ pdmax, int* __restrict__ npiv_out,
-                                                      int64_t nchol0, int64_t maxnchol, double dmin)
+//
+// Every pivot needs all previous vectors of its row and of every other row, so
+// the search is bound by how fast Lb can be re-read, pivot after pivot.  One
+// cluster of kPivCtas blocks holds it: each keeps its rows of Lb (the first jcap
+// vectors) and of the diagonal in shared memory, four lanes a row.  Per pivot
+// one exchange of the blocks' maxima through distributed shared memory (with
+// the reference's tie rule: strict '>' in increasing index order, chol2_BatchMax,
+// TwoStepCholesky_Step1.f90:720-727) and one read of the pivot's row from its owner.
+// About 3.5 us a pivot, most of it the two exchanges; one block that reads Lb back from
+// L2 took 9 ms for a batch of 1000 rows (pivot phase of 10 atoms, 140 AOs: 20.4 -> 9.0 ms;
+// of 12 atoms, 360 AOs with f shells: 115 -> 53 ms).
+constexpr int kPivCtas = 8, kPivThreads = 512, kPivSub = 4, kPivRowsPerPass = kPivThreads / kPivSub;
+
+__device__ __forceinline__ void cluster_barrier()
 {
-    extern __shared__ double sh[];
-    double* prow = sh;                                   // nb
-    double* s_v = sh + nb;                               // 32
-    int* s_i = reinterpret_cast<int*>(s_v + 32);         // 32
-    double maxv; int maxi;
-    block_argmax(Db, nb, maxv, maxi, s_v, s_i);
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// address of this block's shared variable `p` in block `rank` of the cluster
+__device__ __forceinline__ uint32_t cluster_addr(const void* p, int rank)
+{
+    uint32_t r;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"((uint32_t)__cvta_generic_to_shared(p)), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void cluster_store(uint32_t a, double v)
+{
+    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
+}
+__device__ __forceinline__ void cluster_store(uint32_t a, int v)
+{
+    asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+__device__ __forceinline__ double cluster_load(uint32_t a)
+{
+    double v;
+    asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(v) : "r"(a) : "memory");
+    return v;
+}
+
+__global__ void __cluster_dims__(kPivCtas, 1, 1) __launch_bounds__(kPivThreads, 1)
+k_pivot_batch(const double* __restrict__ Mbb, int nb, const double* __restrict__ Db, double* __restrict__ Lb,
+              int* __restrict__ piv, double* __restrict__ pdmax, int* __restrict__ npiv_out, int64_t nchol0,
+              int64_t maxnchol, double dmin, int rpc, int pitch, int jcap)
+{
+    // rows [row0, row0 + nr) of the batch: rpc a block
+    extern __shared__ __align__(16) double sh[];
+    double* prow = sh;                          // nb: the pivot's row of the vectors so far
+    double* Ds = prow + nb;                     // rpc: residual diagonal of the block's rows
+    double* Ls = Ds + rpc;                      // jcap x pitch: vectors of the block's rows
+    __shared__ double x_v[2][kPivCtas];         // the blocks' maxima, alternating between pivots
+    __shared__ int x_i[2][kPivCtas];
+    const int rank = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int row0 = rank * rpc, nr = min(rpc, nb - row0);   // nr <= 0: no rows
+    for (int r = tid; r < nr; r += kPivThreads) Ds[r] = Db[row0 + r];
+    // a warp takes 8 rows of 4 lanes; the lanes of a row take every fourth vector
+    const int sub = lane >> 3, rl = warp * 8 + (lane & 7);
+
+    // maximum over all rows of the batch and its first index, the same in every thread
+    auto argmax = [&](int par, double& bv, int& bi) {
+        __syncthreads();
+        if (warp == 0) {
+            double v = -DBL_MAX;
+            int i = 0x7fffffff;
+            for (int r = lane; r < nr; r += 32)
+                if (better(Ds[r], row0 + r, v, i)) { v = Ds[r]; i = row0 + r; }
+            for (int off = 16; off > 0; off >>= 1) {
+                const double ov = __shfl_xor_sync(0xffffffffu, v, off);
+                const int oi = __shfl_xor_sync(0xffffffffu, i, off);
+                if (better(ov, oi, v, i)) { v = ov; i = oi; }
+            }
+            if (lane < kPivCtas) {
+                cluster_store(cluster_addr(&x_v[par][rank], lane), v);
+                cluster_store(cluster_addr(&x_i[par][rank], lane), i);
+            }
+            __syncwarp();
+        }
+        cluster_barrier();   // the maxima are exchanged, and every block's vectors so far are complete
+        bv = -DBL_MAX;
+        bi = 0x7fffffff;
+#pragma unroll
+        for (int c = 0; c < kPivCtas; ++c)
+            if (better(x_v[par][c], x_i[par][c], bv, bi)) { bv = x_v[par][c]; bi = x_i[par][c]; }
+    };
+
+    double maxv;
+    int maxi;
+    cluster_barrier();   // every block of the cluster runs before its shared memory is written
+    argmax(0, maxv, maxi);
     int j = 0;
-    bool go = (nchol0 < maxnchol) && nb > 0;
+    bool go = (nchol0 < maxnchol) && maxi < nb;
     while (go) {
-        if (threadIdx.x == 0) { piv[j] = maxi; pdmax[j] = maxv; }
-        for (int i = threadIdx.x; i < j; i += blockDim.x) prow[i] = Lb[maxi + (int64_t)nb * i];
+        if (rank == 0 && tid == 0) { piv[j] = maxi; pdmax[j] = maxv; }
+        const int owner = maxi / rpc, orow = maxi - owner * rpc;
+        const int js = min(j, jcap);
+        for (int i = tid; i < js; i += kPivThreads) prow[i] = cluster_load(cluster_addr(Ls + (size_t)i * pitch + orow, owner));
+        for (int i = js + tid; i < j; i += kPivThreads) prow[i] = __ldcg(Lb + maxi + (int64_t)nb * i);
         __syncthreads();
         const double sq = sqrt(maxv);
-        for (int r = threadIdx.x; r < nb; r += blockDim.x) {
-            double s = Mbb[r + (int64_t)nb * maxi];
-            for (int i = 0; i < j; ++i) s -= Lb[r + (int64_t)nb * i] * prow[i];
-            const double l = s / sq;
-            Lb[r + (int64_t)nb * j] = l;
-            Db[r] -= l * l;
+        for (int r = rl; r < rpc; r += kPivRowsPerPass) {   // uniform within a warp up to the row bound
+            const bool on = r < nr;
+            double s0 = 0.0, s1 = 0.0;
+            if (on) {
+                if (sub == 0) s0 = Mbb[row0 + r + (int64_t)nb * maxi];
+                int i = sub;
+                for (; i + kPivSub < js; i += 2 * kPivSub) {
+                    s0 = fma(-Ls[(size_t)i * pitch + r], prow[i], s0);
+                    s1 = fma(-Ls[(size_t)(i + kPivSub) * pitch + r], prow[i + kPivSub], s1);
+                }
+                for (; i < js; i += kPivSub) s0 = fma(-Ls[(size_t)i * pitch + r], prow[i], s0);
+                for (i = js + sub; i < j; i += kPivSub) s1 = fma(-__ldcg(Lb + row0 + r + (int64_t)nb * i), prow[i], s1);
+            }
+            double s = s0 + s1;
+            s += __shfl_xor_sync(0xffffffffu, s, 8);
+            s += __shfl_xor_sync(0xffffffffu, s, 16);
+            if (on && sub == 0) {
+                const double l = s / sq;
+                if (j < jcap) Ls[(size_t)j * pitch + r] = l;
+                __stcg(Lb + row0 + r + (int64_t)nb * j, l);
+                Ds[r] -= l * l;
+            }
         }
-        __syncthreads();
         ++j;
-        block_argmax(Db, nb, maxv, maxi, s_v, s_i);
+        argmax(j & 1, maxv, maxi);
         if (maxv <= dmin) go = false;
         if (j == nb || nchol0 + j == maxnchol) go = false;
     }
-    if (threadIdx.x == 0) *npiv_out = j;
+    if (rank == 0 && tid == 0) *npiv_out = j;
 }
 
 // Lp(j, i) = Lb(piv[j], i): the pivot rows of the new vectors (lower triangular)
@@ -249,9 +311,18 @@ cudaError_t launch_gather_cols(const double* src, int64_t lds, const int* cols, 
 cudaError_t launch_pivot_batch(const double* Mbb, int nb, double* Db, double* Lb, int* piv, double* pdmax,
                                int* npiv, int64_t nchol0, int64_t maxnchol, double dmin, cudaStream_t s)
 {
-    const size_t smem = sizeof(double) * (size_t)(nb + 32) + sizeof(int) * 32;
-    if (smem > 48 * 1024) cudaFuncSetAttribute(k_pivot_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_pivot_batch<<<1, 1024, smem, s>>>(Mbb, nb, Db, Lb, piv, pdmax, npiv, nchol0, maxnchol, dmin);
+    // rows a block (a multiple of a warp's 8); the pitch 8 mod 16 keeps the four lanes of a row
+    // and the eight rows of a warp in different banks; as many vectors as fit 200 KB
+    const int rpc = std::max(8, ((nb + kPivCtas - 1) / kPivCtas + 7) / 8 * 8);
+    const int pitch = (rpc + 15) / 16 * 16 + 8;
+    const int64_t room = (int64_t)(200 * 1024) / 8 - nb - rpc;
+    const int jcap = room > 0 ? (int)std::min<int64_t>(nb, room / pitch) : 0;
+    const size_t smem = sizeof(double) * ((size_t)nb + rpc + (size_t)jcap * pitch);
+    // the same value from every caller: workers of a batch launch at the same time
+    cudaError_t e = cudaFuncSetAttribute(k_pivot_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024);
+    if (e != cudaSuccess) return e;
+    k_pivot_batch<<<kPivCtas, kPivThreads, smem, s>>>(Mbb, nb, Db, Lb, piv, pdmax, npiv, nchol0, maxnchol, dmin, rpc,
+                                                      pitch, jcap);
     count_launch();
     return cudaGetLastError();
 }
