@@ -6,10 +6,11 @@
 //    c[i sci + j scj]), an optional batch index, and structure flags that skip
 //    the zero half of a triangular operand (the K range of a tile shrinks) or
 //    the strictly upper tiles of a symmetric update.  128 x 128 tiles, 8 warps
-//    of 64 x 32, K in blocks of 16 through a three-stage ring of shared
-//    buffers filled by cp.async (two blocks in flight during the products).
+//    of 64 x 32 (or 64 x 64 tiles, 4 warps of 32 x 32, for small products), K in
+//    blocks of 16 through a three-stage ring of shared buffers filled by cp.async
+//    (two blocks in flight during the products).
 //  * k_potrf_leaf: Cholesky factor and inverse of one diagonal block of at
-//    most 64 rows in shared memory.
+//    most 64 rows, in the registers of a warp by halves.
 //  * k_trsm_leaf: X = B L^-T for a block of at most 32 columns, one row of B
 //    per thread, by forward substitution.
 //
@@ -26,13 +27,20 @@
 
 namespace gci {
 
-constexpr int kDgBM = 128, kDgBN = 128, kDgBK = 16, kDgThreads = 256, kDgStages = 3;
-// Shared K slice of one operand: [kDgBK][kDgLdR] when its contiguous global index is the row
-// index (i or j), [128][kDgLdK] when it is l.  Both paddings make the fragment loads of a
-// half-warp conflict-free.
-constexpr int kDgLdR = kDgBM + 4, kDgLdK = kDgBK + 4;
-constexpr int kDgTile = kDgBM * kDgLdK > kDgBK * kDgLdR ? kDgBM * kDgLdK : kDgBK * kDgLdR;   // doubles
-constexpr int kDgSmem = kDgStages * 2 * kDgTile * (int)sizeof(double);
+// Tile shapes of k_dgemm: BT x BT output tile, WM x WN per warp.  Shared K slice of one operand:
+// [BK][LdR] when its contiguous global index is the row index (i or j), [BT][LdK] when it is l.
+// Both paddings make the fragment loads of a half-warp conflict-free.
+template <int BT, int WM_, int WN_>
+struct DgShape {
+    static constexpr int B = BT, WM = WM_, WN = WN_, BK = 16, STAGES = 3;
+    static constexpr int WARPS_M = BT / WM, THREADS = 32 * WARPS_M * (BT / WN);
+    static constexpr int LdR = BT + 4, LdK = BK + 4;
+    static constexpr int TILE = BT * LdK > BK * LdR ? BT * LdK : BK * LdR;   // doubles
+    static constexpr int SMEM = STAGES * 2 * TILE * (int)sizeof(double);
+    static constexpr int COPIES = BT * BK / THREADS;   // per thread, operand and K block
+};
+using DgLarge = DgShape<128, 64, 32>;
+using DgSmall = DgShape<64, 32, 32>;
 constexpr int kLeafN = 64, kLeafLd = kLeafN + 1;
 constexpr int kTrsmW = 32;
 
@@ -53,37 +61,39 @@ __device__ __forceinline__ void cp_async8(double* dst, const double* src, int sr
 
 // AK: A's contiguous global index is l (sal == 1), else i; BK: B's is l (sbl == 1), else j.
 // Each operand is copied along its contiguous index into the matching shared layout.
-template <bool AK, bool BK>
-__global__ void __launch_bounds__(kDgThreads, 1) k_dgemm(const DgemmArgs p)
+template <class S, bool AK, bool BK>
+__global__ void __launch_bounds__(S::THREADS, 1) k_dgemm(const DgemmArgs p)
 {
+    constexpr int BT = S::B, BKD = S::BK, LdR = S::LdR, LdK = S::LdK, TILE = S::TILE, STAGES = S::STAGES;
+    constexpr int MT = S::WM / 8, NT = S::WN / 8;
     extern __shared__ __align__(16) double dg_smem[];
-    const int64_t m0 = (int64_t)blockIdx.x * kDgBM, n0 = (int64_t)blockIdx.y * kDgBN;
-    if ((p.flags & kDgCLower) && n0 >= m0 + kDgBM) return;   // tile strictly above the diagonal
+    const int64_t m0 = (int64_t)blockIdx.x * BT, n0 = (int64_t)blockIdx.y * BT;
+    if ((p.flags & kDgCLower) && n0 >= m0 + BT) return;   // tile strictly above the diagonal
     const double* A = p.a + (int64_t)blockIdx.z * p.sab;
     const double* B = p.b + (int64_t)blockIdx.z * p.sbb;
     double* Cm = p.c + (int64_t)blockIdx.z * p.scb;
     int64_t klo = 0, khi = p.k;
-    if (p.flags & kDgALower) khi = min(khi, m0 + kDgBM);   // A(i, l) = 0 for l > i
-    if (p.flags & kDgBUpper) khi = min(khi, n0 + kDgBN);   // B(l, j) = 0 for l > j
+    if (p.flags & kDgALower) khi = min(khi, m0 + BT);   // A(i, l) = 0 for l > i
+    if (p.flags & kDgBUpper) khi = min(khi, n0 + BT);   // B(l, j) = 0 for l > j
     if (p.flags & kDgBLower) klo = max(klo, n0);           // B(l, j) = 0 for l < j
-    const int64_t nkt = khi > klo ? (khi - klo + kDgBK - 1) / kDgBK : 0;
+    const int64_t nkt = khi > klo ? (khi - klo + BKD - 1) / BKD : 0;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int wm = warp & 1, wn = warp >> 1;
+    const int wm = warp % S::WARPS_M, wn = warp / S::WARPS_M;
     // copy s of this thread: tile row r + s dr, tile k kq + s dk
-    const int a_r = AK ? tid >> 4 : tid & 127, a_k = AK ? tid & 15 : tid >> 7;
-    const int b_r = BK ? tid >> 4 : tid & 127, b_k = BK ? tid & 15 : tid >> 7;
-    constexpr int a_dr = AK ? 16 : 0, a_dk = AK ? 0 : 2;
-    constexpr int b_dr = BK ? 16 : 0, b_dk = BK ? 0 : 2;
-    auto a_off = [](int r, int k) { return AK ? r * kDgLdK + k : k * kDgLdR + r; };
-    auto b_off = [](int r, int k) { return BK ? r * kDgLdK + k : k * kDgLdR + r; };
+    const int a_r = AK ? tid / BKD : tid % BT, a_k = AK ? tid % BKD : tid / BT;
+    const int b_r = BK ? tid / BKD : tid % BT, b_k = BK ? tid % BKD : tid / BT;
+    constexpr int a_dr = AK ? S::THREADS / BKD : 0, a_dk = AK ? 0 : S::THREADS / BT;
+    constexpr int b_dr = BK ? S::THREADS / BKD : 0, b_dk = BK ? 0 : S::THREADS / BT;
+    auto a_off = [](int r, int k) { return AK ? r * LdK + k : k * LdR + r; };
+    auto b_off = [](int r, int k) { return BK ? r * LdK + k : k * LdR + r; };
     auto issue = [&](int64_t kt) {
         if (kt < nkt) {
-            const int64_t k0 = klo + kt * kDgBK;
-            double* as = dg_smem + (kt % kDgStages) * 2 * kDgTile;
-            double* bs = as + kDgTile;
+            const int64_t k0 = klo + kt * BKD;
+            double* as = dg_smem + (kt % STAGES) * 2 * TILE;
+            double* bs = as + TILE;
 #pragma unroll
-            for (int s = 0; s < 8; ++s) {
+            for (int s = 0; s < S::COPIES; ++s) {
                 const int ra = a_r + s * a_dr, ka = a_k + s * a_dk;
                 const int64_t i = m0 + ra, l = k0 + ka;
                 const bool va = i < p.m && l < khi;
@@ -97,47 +107,47 @@ __global__ void __launch_bounds__(kDgThreads, 1) k_dgemm(const DgemmArgs p)
         asm volatile("cp.async.commit_group;" ::: "memory");   // one group per tile, empty past the end
     };
 
-    double acc[8][4][2];
+    double acc[MT][NT][2];
 #pragma unroll
-    for (int mt = 0; mt < 8; ++mt)
+    for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
-        for (int nt = 0; nt < 4; ++nt) acc[mt][nt][0] = acc[mt][nt][1] = 0.0;
+        for (int nt = 0; nt < NT; ++nt) acc[mt][nt][0] = acc[mt][nt][1] = 0.0;
 
 #pragma unroll
-    for (int s = 0; s < kDgStages - 1; ++s) issue(s);
+    for (int s = 0; s < STAGES - 1; ++s) issue(s);
 #pragma unroll 1
     for (int64_t kt = 0; kt < nkt; ++kt) {
-        asm volatile("cp.async.wait_group %0;" ::"n"(kDgStages - 2) : "memory");   // tile kt has landed
+        asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");   // tile kt has landed
         __syncthreads();   // every thread's copies of tile kt; every warp done with tile kt - 1
-        issue(kt + kDgStages - 1);
-        const double* as = dg_smem + (kt % kDgStages) * 2 * kDgTile;
-        const double* bs = as + kDgTile;
+        issue(kt + STAGES - 1);
+        const double* as = dg_smem + (kt % STAGES) * 2 * TILE;
+        const double* bs = as + TILE;
 #pragma unroll
-        for (int kk = 0; kk < kDgBK / 4; ++kk) {
+        for (int kk = 0; kk < BKD / 4; ++kk) {
             const int kq = kk * 4 + (lane & 3);
-            double af[8], bf[4];
+            double af[MT], bf[NT];
 #pragma unroll
-            for (int mt = 0; mt < 8; ++mt) af[mt] = as[a_off(wm * 64 + mt * 8 + (lane >> 2), kq)];
+            for (int mt = 0; mt < MT; ++mt) af[mt] = as[a_off(wm * S::WM + mt * 8 + (lane >> 2), kq)];
 #pragma unroll
-            for (int nt = 0; nt < 4; ++nt) bf[nt] = bs[b_off(wn * 32 + nt * 8 + (lane >> 2), kq)];
+            for (int nt = 0; nt < NT; ++nt) bf[nt] = bs[b_off(wn * S::WN + nt * 8 + (lane >> 2), kq)];
 #pragma unroll
-            for (int mt = 0; mt < 8; ++mt)
+            for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
-                for (int nt = 0; nt < 4; ++nt) dmma(acc[mt][nt], af[mt], bf[nt]);
+                for (int nt = 0; nt < NT; ++nt) dmma(acc[mt][nt], af[mt], bf[nt]);
         }
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
 
     // D fragment: lane l holds D(l / 4, 2 (l % 4) + e)
 #pragma unroll
-    for (int mt = 0; mt < 8; ++mt) {
-        const int64_t i = m0 + wm * 64 + mt * 8 + (lane >> 2);
+    for (int mt = 0; mt < MT; ++mt) {
+        const int64_t i = m0 + wm * S::WM + mt * 8 + (lane >> 2);
         if (i >= p.m) continue;
 #pragma unroll
-        for (int nt = 0; nt < 4; ++nt)
+        for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
-                const int64_t j = n0 + wn * 32 + nt * 8 + 2 * (lane & 3) + e;
+                const int64_t j = n0 + wn * S::WN + nt * 8 + 2 * (lane & 3) + e;
                 if (j >= p.n || ((p.flags & kDgCLower) && j > i)) continue;
                 double* cp = Cm + i * p.sci + j * p.scj;
                 const double v = p.alpha * acc[mt][nt][e];
@@ -146,63 +156,144 @@ __global__ void __launch_bounds__(kDgThreads, 1) k_dgemm(const DgemmArgs p)
     }
 }
 
-cudaError_t dgemm(const DgemmArgs& p, int64_t batch, cudaStream_t st)
+template <class S>
+static cudaError_t dgemm_launch(const DgemmArgs& p, int64_t batch, cudaStream_t st)
 {
-    if (p.m <= 0 || p.n <= 0 || batch <= 0) return cudaSuccess;
-    const int64_t gm = (p.m + kDgBM - 1) / kDgBM, gn = (p.n + kDgBN - 1) / kDgBN;
+    const int64_t gm = (p.m + S::B - 1) / S::B, gn = (p.n + S::B - 1) / S::B;
     if (gm > 0x7fffffffLL || gn > 65535 || batch > 65535) return cudaErrorInvalidValue;
     const bool ak = p.sal == 1 && p.sai != 1, bk = p.sbl == 1 && p.sbj != 1;
-    auto fn = ak ? (bk ? k_dgemm<true, true> : k_dgemm<true, false>) : (bk ? k_dgemm<false, true> : k_dgemm<false, false>);
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kDgSmem);
+    auto fn = ak ? (bk ? k_dgemm<S, true, true> : k_dgemm<S, true, false>)
+                 : (bk ? k_dgemm<S, false, true> : k_dgemm<S, false, false>);
+    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, S::SMEM);
     if (e != cudaSuccess) return e;
-    fn<<<dim3((unsigned)gm, (unsigned)gn, (unsigned)batch), kDgThreads, kDgSmem, st>>>(p);
+    fn<<<dim3((unsigned)gm, (unsigned)gn, (unsigned)batch), S::THREADS, S::SMEM, st>>>(p);
     count_launch();
     return cudaGetLastError();
 }
 
+// 128 x 128 tiles where they give every SM one (half of them count in a lower-triangular update);
+// below that 64 x 64 tiles, whose four times as many blocks finish earlier although each product
+// reads its operands twice as often (1003 x 257 x 300: 91 -> 43 us).  Every element sums its
+// products in the same order in both.
+cudaError_t dgemm(const DgemmArgs& p, int64_t batch, cudaStream_t st)
+{
+    if (p.m <= 0 || p.n <= 0 || batch <= 0) return cudaSuccess;
+    int64_t tiles = ((p.m + 127) / 128) * ((p.n + 127) / 128) * batch;
+    if (p.flags & kDgCLower) tiles = (tiles + 1) / 2;
+    const bool small = tiles < 148 && (p.n + 63) / 64 <= 65535;
+    return small ? dgemm_launch<DgSmall>(p, batch, st) : dgemm_launch<DgLarge>(p, batch, st);
+}
+
 // ------------------------------------------------------------------ leaves
+// Cholesky factor and inverse of the 32 x 32 block at S (lower part, pitch kLeafLd) by one warp,
+// lane = row: the row lives in registers, column j reaches the other rows by shuffles.  The
+// inverse (lane = column) by right-looking substitution, L broadcast from shared memory.  Returns
+// the first non-positive pivot + 1, or 0.
+__device__ static int leaf_block(double* S, double* X, int lane)
+{
+    double r[32], invd = 0.0;
+    int bad = 0;
+#pragma unroll
+    for (int k = 0; k < 32; ++k) r[k] = S[lane * kLeafLd + k];
+#pragma unroll
+    for (int j = 0; j < 32; ++j) {
+        const double d = __shfl_sync(0xffffffffu, r[j], j);   // the same value in every lane
+        if (!(d > 0.0) && !bad) bad = j + 1;
+        const double sq = sqrt(d), inv = 1.0 / sq;
+        if (lane == j) invd = inv;
+        r[j] = lane == j ? sq : r[j] * inv;
+#pragma unroll
+        for (int k = j + 1; k < 32; ++k) r[k] = fma(-r[j], __shfl_sync(0xffffffffu, r[j], k), r[k]);
+    }
+    if (bad) return bad;
+#pragma unroll
+    for (int k = 0; k < 32; ++k)
+        if (k <= lane) S[lane * kLeafLd + k] = r[k];
+    __syncwarp();
+    double x[32];
+#pragma unroll
+    for (int i = 0; i < 32; ++i) x[i] = i == lane ? 1.0 : 0.0;
+#pragma unroll
+    for (int i = 0; i < 32; ++i) {
+        x[i] *= __shfl_sync(0xffffffffu, invd, i);
+        X[i * kLeafLd + lane] = x[i];   // zero above the diagonal
+#pragma unroll
+        for (int k = i + 1; k < 32; ++k) x[k] = fma(-S[k * kLeafLd + i], x[i], x[k]);
+    }
+    return 0;
+}
+
 // Diagonal block [off, off + n) of a (n <= 64): L (lower part of a) and X = L^-1 (x, zeros
 // above the diagonal).  A non-positive pivot j sets *info = off + j + 1 (first failure kept).
-__global__ void __launch_bounds__(128) k_potrf_leaf(double* a, double* x, int64_t ld, int64_t off, int n, int* info)
+// Two 32-row halves, each factored and inverted by one warp in registers, joined by 32 x 32
+// products over the block (L21 = A21 X11^T, A22 -= L21 L21^T, X21 = -X22 L21 X11).  Bound by the
+// latency of the 64 columns' square roots, quotients and exchanges.  A chain of 64 columns of
+// shared-memory updates with three barriers each is several times longer: with the smaller GEMM
+// tiles, factor and inverse of 501 rows 1.93 -> 0.80 ms, of 4001 rows 20.5 -> 9.5 ms.
+__global__ void __launch_bounds__(256) k_potrf_leaf(double* a, double* x, int64_t ld, int64_t off, int n, int* info)
 {
     extern __shared__ double lf_smem[];
     double* S = lf_smem;                       // [kLeafN][kLeafLd]
     double* X = lf_smem + kLeafN * kLeafLd;    // [kLeafN][kLeafLd]
-    const int tid = threadIdx.x;
-    for (int idx = tid; idx < n * n; idx += blockDim.x) {
-        const int i = idx % n, j = idx / n;
-        S[i * kLeafLd + j] = i >= j ? a[(off + i) + (off + j) * ld] : 0.0;
+    __shared__ int s_bad;
+    constexpr int H = kLeafN / 2;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    // rows past n continue as the identity
+    for (int idx = tid; idx < kLeafN * kLeafN; idx += 256) {
+        const int i = idx % kLeafN, j = idx / kLeafN;
+        S[i * kLeafLd + j] = i < n && j <= i ? a[(off + i) + (off + j) * ld] : (i == j ? 1.0 : 0.0);
     }
     __syncthreads();
-    for (int j = 0; j < n; ++j) {
-        const double d = S[j * kLeafLd + j];   // the same value in every thread: a uniform branch
-        if (!(d > 0.0)) {
-            if (tid == 0) atomicCAS(info, 0, (int)(off + j + 1));
+    if (warp == 0) {
+        const int bad = leaf_block(S, X, lane);
+        if (lane == 0) s_bad = bad;
+    }
+    __syncthreads();
+    if (s_bad) {
+        if (tid == 0) atomicCAS(info, 0, (int)(off + s_bad));
+        return;
+    }
+    if (n > H) {
+        // thread: row lane of the lower half, columns warp + 8 q
+        double acc[4];
+        const double* A21 = S + (H + lane) * kLeafLd;
+        auto product = [&](const double* row, auto right) {   // sum_k row[k] right(k, column)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) acc[q] = 0.0;
+            for (int k = 0; k < H; ++k) {
+                const double v = row[k];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) acc[q] = fma(v, right(k, warp + 8 * q), acc[q]);
+            }
+            __syncthreads();   // every operand has been read
+        };
+        product(A21, [&](int k, int j) { return X[j * kLeafLd + k]; });                    // L21 = A21 X11^T
+#pragma unroll
+        for (int q = 0; q < 4; ++q) S[(H + lane) * kLeafLd + warp + 8 * q] = acc[q];
+        __syncthreads();
+        product(A21, [&](int k, int j) { return S[(H + j) * kLeafLd + k]; });              // A22 -= L21 L21^T
+#pragma unroll
+        for (int q = 0; q < 4; ++q) S[(H + lane) * kLeafLd + H + warp + 8 * q] -= acc[q];
+        __syncthreads();
+        if (warp == 0) {
+            const int bad = leaf_block(S + H * kLeafLd + H, X + H * kLeafLd + H, lane);
+            if (lane == 0) s_bad = bad ? H + bad : 0;
+        }
+        __syncthreads();
+        if (s_bad) {
+            if (tid == 0) atomicCAS(info, 0, (int)(off + s_bad));
             return;
         }
-        const double r = sqrt(d);
+        product(A21, [&](int k, int j) { return X[k * kLeafLd + j]; });                    // T = L21 X11
+#pragma unroll
+        for (int q = 0; q < 4; ++q) X[lane * kLeafLd + H + warp + 8 * q] = acc[q];        // (above the diagonal of X)
         __syncthreads();
-        for (int i = j + tid; i < n; i += blockDim.x) S[i * kLeafLd + j] = i == j ? r : S[i * kLeafLd + j] / r;
-        __syncthreads();
-        const int t = n - j - 1;
-        for (int idx = tid; idx < t * t; idx += blockDim.x) {
-            const int i = j + 1 + idx % t, k = j + 1 + idx / t;
-            if (k <= i) S[i * kLeafLd + k] -= S[i * kLeafLd + j] * S[k * kLeafLd + j];
-        }
+        product(X + (H + lane) * kLeafLd + H, [&](int k, int j) { return X[k * kLeafLd + H + j]; });
+#pragma unroll
+        for (int q = 0; q < 4; ++q) X[(H + lane) * kLeafLd + warp + 8 * q] = -acc[q];      // X21 = -X22 T
         __syncthreads();
     }
-    // X = L^-1 column by column: X(c, c) = 1 / L(c, c), X(i, c) = -sum_{c <= k < i} L(i, k) X(k, c) / L(i, i)
-    if (tid < n) {
-        const int c = tid;
-        X[c * kLeafLd + c] = 1.0 / S[c * kLeafLd + c];
-        for (int i = c + 1; i < n; ++i) {
-            double s = 0.0;
-            for (int k = c; k < i; ++k) s = fma(S[i * kLeafLd + k], X[k * kLeafLd + c], s);
-            X[i * kLeafLd + c] = -s / S[i * kLeafLd + i];
-        }
-    }
-    __syncthreads();
-    for (int idx = tid; idx < n * n; idx += blockDim.x) {
+    for (int idx = tid; idx < n * n; idx += 256) {
         const int i = idx % n, j = idx / n;
         if (i >= j) a[(off + i) + (off + j) * ld] = S[i * kLeafLd + j];
         x[(off + i) + (off + j) * ld] = i >= j ? X[i * kLeafLd + j] : 0.0;
@@ -253,7 +344,7 @@ static DgemmArgs dg(int64_t m, int64_t n, int64_t k, double alpha, const double*
 static cudaError_t potrf_rec(double* a, double* x, int64_t ld, int64_t off, int64_t n, int* info, cudaStream_t st)
 {
     if (n <= kLeafN) {
-        k_potrf_leaf<<<1, 128, 2 * kLeafN * kLeafLd * sizeof(double), st>>>(a, x, ld, off, (int)n, info);
+        k_potrf_leaf<<<1, 256, 2 * kLeafN * kLeafLd * sizeof(double), st>>>(a, x, ld, off, (int)n, info);
         count_launch();
         return cudaGetLastError();
     }
