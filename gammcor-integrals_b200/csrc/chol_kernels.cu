@@ -259,6 +259,23 @@ __global__ void k_zero_upper(double* __restrict__ A, int64_t n)
     }
 }
 
+// A(i, j) = A(j, i) where rank[i] > rank[j], through 32 x 32 tiles in shared memory so that both
+// sides are read and written in runs (bound by HBM: half of A read, half written).
+__global__ void __launch_bounds__(256) k_mirror(double* __restrict__ A, int64_t ld, int64_t n,
+                                                const int* __restrict__ rank)
+{
+    __shared__ double t[32][33];
+    const int64_t i0 = (int64_t)blockIdx.x * 32, j0 = (int64_t)blockIdx.y * 32;   // destination tile A(i0.., j0..)
+    const int x = threadIdx.x & 31, y = threadIdx.x >> 5;
+    for (int k = y; k < 32; k += 8)
+        if (j0 + x < n && i0 + k < n) t[k][x] = A[(j0 + x) + ld * (i0 + k)];
+    __syncthreads();
+    for (int k = y; k < 32; k += 8) {
+        const int64_t i = i0 + x, j = j0 + k;
+        if (i < n && j < n && __ldg(rank + i) > __ldg(rank + j)) A[i + ld * j] = t[x][k];
+    }
+}
+
 // Unpack Rkpq(k, pq) (k in [k0, k0+kc)) into the dense symmetric AO-pair
 // layout U[p][q][k - k0] (both triangles) for the AO->MO GEMMs.
 // One entry per stored orbital pair: pq_ao[2*i] = p, pq_ao[2*i+1] = q, and
@@ -350,6 +367,15 @@ cudaError_t launch_downdate(double* D, const double* L, int64_t ld, int64_t n, i
 cudaError_t launch_max(const double* v, int64_t n, double* out, cudaStream_t s)
 {
     k_max<<<1, 1024, 0, s>>>(v, n, out);
+    count_launch();
+    return cudaGetLastError();
+}
+cudaError_t launch_mirror(double* A, int64_t ld, int64_t n, const int* rank, cudaStream_t s)
+{
+    if (n <= 0) return cudaSuccess;
+    const unsigned g = (unsigned)((n + 31) / 32);
+    if (g > 65535) return cudaErrorInvalidValue;
+    k_mirror<<<dim3(g, g), 256, 0, s>>>(A, ld, n, rank);
     count_launch();
     return cudaGetLastError();
 }

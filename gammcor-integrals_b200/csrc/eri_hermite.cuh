@@ -40,6 +40,8 @@
 #pragma once
 #include "gci_common.h"
 #include "boys.cuh"
+#include <algorithm>
+#include <atomic>
 #include <type_traits>
 
 namespace gci {
@@ -195,10 +197,10 @@ __device__ __noinline__ void hm_produce(const double* __restrict__ Bp, const dou
     const double PQ = P * Q;
     const double den = P + Q + kappa * PQ;
     const double alpha = PQ / den;
-    const double pref = on ? 34.986836655249725 / (PQ * sqrt(den)) : 0.0;
+    const double pref = 34.986836655249725 / (PQ * sqrt(den));
     double F[LT + 1];
     boys_fm<LT>(alpha * (dx * dx + dy * dy + dz * dz), boys, F);
-    double pw = pref;
+    double pw = on ? pref : 0.0;
     const double m2a = -2.0 * alpha;
 #pragma unroll
     for (int m = 0; m <= LT; ++m) { F[m] *= pw; pw *= m2a; }
@@ -249,13 +251,20 @@ k_eri_hm(const HmArgs a)
     // Hankel fragment (m, ks) of a unit: lane l reads R_{il,kl}(h + g) with (il, h) = 8 m + l/4 and
     // (kl, g) = 4 ks + l%4 flattened over the unit's rows and columns.  Padding reads entry 0 (a
     // finite value): its column vectors or its row vectors are zero.
+    // (t | u << 8 | v << 16 of the Hermite indices first, where the warps' data will be)
+    int* herm = reinterpret_cast<int*>(smem);
+    constexpr int HMAX = S::H1 > S::H2 ? S::H1 : S::H2;
+    static_assert(HMAX * sizeof(int) <= sizeof(double) * S::WARPS * S::WS, "index list");
+    for (int h = threadIdx.x; h < HMAX; h += S::TPB) herm[h] = herm_t(h) | (herm_u(h) << 8) | (herm_v(h) << 16);
+    __syncthreads();
     for (int c = threadIdx.x; c < S::TAB; c += S::TPB) {
         const int m = c % S::MTP, l = (c / S::MTP) & 31, ks = c / (S::MTP * 32);
         const int rho = 8 * m + (l >> 2), kap = 4 * ks + (l & 3);
         int off = 0;
         if (rho < IB * S::H1 && kap < KP * S::H2) {
             const int il = rho / S::H1, h = rho - il * S::H1, kl = kap / S::H2, g = kap - kl * S::H2;
-            off = 8 * ((il * KP + kl) * S::QS + hm_ridx(LT, herm_t(h) + herm_t(g), herm_u(h) + herm_u(g), herm_v(h) + herm_v(g)));
+            const int tuv = herm[h] + herm[g];   // no carries: components stay below 256
+            off = 8 * ((il * KP + kl) * S::QS + hm_ridx(LT, tuv & 255, (tuv >> 8) & 255, tuv >> 16));
         }
         tab[c] = (unsigned short)off;
     }
@@ -266,21 +275,25 @@ k_eri_hm(const HmArgs a)
     const uint32_t ring_s = (uint32_t)__cvta_generic_to_shared(ring);
     __syncthreads();
 
-    const int64_t ntasks = a.nrows * a.nchunks;
+    const int64_t nparts = a.nrows * a.nchunks * a.split;
     for (;;) {
         // tasks in row-major order (a row pair's chunks are consecutive), taken
-        // one at a time from the launch's counter
+        // one (or one part) at a time from the launch's counter
         unsigned long long t0 = 0;
         if (lane == 0) t0 = atomicAdd(a.counter, 1ULL);
-        const int64_t task = (int64_t)__shfl_sync(0xffffffffu, t0, 0);
-        if (task >= ntasks) break;
+        const int64_t tpart = (int64_t)__shfl_sync(0xffffffffu, t0, 0);
+        if (tpart >= nparts) break;
+        const int64_t task = tpart / a.split;
+        const int part = (int)(tpart - task * a.split);
         const int64_t rix = task / a.nchunks;
         const HmChunk ch = a.chunks[a.chunk_ids[task - rix * a.nchunks]];
         const int rp = a.rows[rix];
+        if (a.upper && ch.pair < rp) continue;   // the mirror image of another task
         const ShellPairDev pr = a.pairs[rp];
         const ShellPairDev pc = a.pairs[ch.pair];
         const int nb = pr.npp, nk = pc.npp;
-        const int nib = (nb + IB - 1) / IB, nkg = (nk + KP - 1) / KP, nu = nib * nkg;
+        const int nib = (nb + IB - 1) / IB, nkg = (nk + KP - 1) / KP;
+        const int ib0 = nib * part / a.split, nu = (nib * (part + 1) / a.split - ib0) * nkg;
         const int rsr = pp_record(pr.l1, pr.l2), rsc = pp_record(pc.l1, pc.l2);
         const double* __restrict__ rrec = a.pp + pr.rec_off;
         const double* __restrict__ crec = a.pp + pc.rec_off;
@@ -316,7 +329,7 @@ k_eri_hm(const HmArgs a)
         for (int m = 0; m < MT; ++m)
 #pragma unroll
             for (int n = 0; n < NT; ++n) X[m][n][0] = X[m][n][1] = 0.0;
-        int ib = 0, kg = 0;   // block and group of the unit whose products come next
+        int ib = ib0, kg = 0;   // block and group of the unit whose products come next
 
         for (int u0 = 0; u0 < nu; u0 += UB) {
             const int un = nu - u0 < UB ? nu - u0 : UB;
@@ -326,7 +339,7 @@ k_eri_hm(const HmArgs a)
             for (int q = lane / S::SL; q < un * UQ; q += 32 / S::SL) {
                 const int ul = q / UQ, rq = q - ul * UQ;
                 const int u = u0 + ul, uib = u / nkg, ukg = u - uib * nkg;
-                int i = uib * IB + rq / KP, k = ukg * KP + rq % KP;
+                int i = (ib0 + uib) * IB + rq / KP, k = ukg * KP + rq % KP;
                 const int on = i < nb && k < nk;
                 if (!on) i = k = 0;
                 hm_produce<LT, S::SL>(rrec + (size_t)i * rsr, crec + (size_t)k * rsc, a.kappa, a.boys, on,
@@ -436,6 +449,31 @@ k_eri_hm(const HmArgs a)
         }
         asm volatile("cp.async.wait_group 0;" ::: "memory");
 
+        if (a.split > 1) {
+            const int used = (nR + 7) / 8 * NT * 64;
+            double* pt = a.part + task * a.split * S::OS;
+            if (nu > 0)
+                for (int w = 2 * lane; w < used; w += 64)
+                    __stcg(reinterpret_cast<double2*>(pt + part * S::OS + w), *reinterpret_cast<const double2*>(Os + w));
+            __threadfence();
+            __syncwarp();
+            int last = 0;
+            if (lane == 0) last = atomicAdd(a.arrive + task, 1) == a.split - 1;
+            if (!__shfl_sync(0xffffffffu, last, 0)) continue;
+            __threadfence();
+            for (int w = 2 * lane; w < used; w += 64) {
+                double2 sum = make_double2(0.0, 0.0);
+                for (int q = 0; q < a.split; ++q) {
+                    // a part without blocks, or a task without column primitive pairs, left nothing
+                    if (nkg == 0 || nib * q / a.split == nib * (q + 1) / a.split) continue;
+                    const double2 v = __ldcg(reinterpret_cast<const double2*>(pt + q * S::OS + w));
+                    sum.x += v.x;
+                    sum.y += v.y;
+                }
+                *reinterpret_cast<double2*>(Os + w) = sum;
+            }
+        }
+
         // scatter: element (m, n, l, e) of the block is O(8 m + l/4, 8 n + 2 (l%4) + e)
 #pragma unroll 1
         for (int m = 0; m < MTO; ++m) {
@@ -468,54 +506,86 @@ k_eri_hm(const HmArgs a)
 
 namespace gci {
 
-using HmLaunchFn = cudaError_t (*)(const HmArgs&, cudaStream_t);
+// How a class is launched: warps resident at once on the device (0: a CUDA error), doubles of
+// a task's output block, and the launch itself.
+struct HmLaunch {
+    cudaError_t (*launch)(const HmArgs&, cudaStream_t);
+    int (*resident)();
+    int block;
+};
 
 // The shared-memory attribute is set on every launch: it belongs to the
 // current device, and the library may be called on several devices.
 template <int L1, int L2, int NT>
+static cudaError_t hm_prepare()
+{
+    return cudaFuncSetAttribute(k_eri_hm<L1, L2, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)HmShape<L1, L2, NT>::smem_bytes());
+}
+
+// Blocks resident at once: a property of the kernel and of the sm_100a GPU it is built for, the
+// same on every device, so it is asked once.
+template <int L1, int L2, int NT>
+static int hm_resident_blocks()
+{
+    using S = HmShape<L1, L2, NT>;
+    static std::atomic<int> known{0};
+    int n = known.load(std::memory_order_relaxed);
+    if (n > 0) return n;
+    int dev = 0, nsm = 0, per_sm = 0;
+    if (hm_prepare<L1, L2, NT>() != cudaSuccess || cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_eri_hm<L1, L2, NT>, S::TPB, S::smem_bytes()) !=
+            cudaSuccess)
+        return 0;
+    n = nsm * (per_sm < 1 ? 1 : per_sm);
+    known.store(n, std::memory_order_relaxed);
+    return n;
+}
+
+template <int L1, int L2, int NT>
+static int hm_resident()
+{
+    return hm_resident_blocks<L1, L2, NT>() * HmShape<L1, L2, NT>::WARPS;
+}
+
+template <int L1, int L2, int NT>
 static cudaError_t launch_hm(const HmArgs& a, cudaStream_t st)
 {
     using S = HmShape<L1, L2, NT>;
-    const int64_t ntasks = a.nrows * a.nchunks;
-    if (ntasks <= 0) return cudaSuccess;
-    auto kern = k_eri_hm<L1, L2, NT>;
-    const size_t smem = S::smem_bytes();
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const int64_t nparts = a.nrows * a.nchunks * a.split;
+    if (nparts <= 0) return cudaSuccess;
+    cudaError_t e = hm_prepare<L1, L2, NT>();
     if (e != cudaSuccess) return e;
     // persistent: as many blocks as are resident at once; warps take tasks from a.counter
-    int dev = 0, nsm = 0, per_sm = 0;
-    if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
-    if ((e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, S::TPB, smem)) != cudaSuccess) return e;
-    if (per_sm < 1) per_sm = 1;
-    int64_t blocks = (ntasks + S::WARPS - 1) / S::WARPS;
-    const int64_t cap = (int64_t)nsm * per_sm;
-    if (blocks > cap) blocks = cap;
-    kern<<<(unsigned)blocks, S::TPB, smem, st>>>(a);
+    const int64_t cap = hm_resident_blocks<L1, L2, NT>();
+    if (cap <= 0) return cudaErrorInvalidDevice;
+    const int64_t blocks = std::min<int64_t>((nparts + S::WARPS - 1) / S::WARPS, cap);
+    k_eri_hm<L1, L2, NT><<<(unsigned)blocks, S::TPB, S::smem_bytes(), st>>>(a);
     return cudaGetLastError();
 }
 
 // tab[L1][L2][NT - 1] for L2 = 0 .. kMaxPairL and NT = 1 .. hm_max_nt(L1)
 template <int L1, int L2, int NT = 1>
-static void register_hm_nt(HmLaunchFn (*tab)[kMaxPairL + 1][kHmMaxNT])
+static void register_hm_nt(HmLaunch (*tab)[kMaxPairL + 1][kHmMaxNT])
 {
-    tab[L1][L2][NT - 1] = &launch_hm<L1, L2, NT>;
+    tab[L1][L2][NT - 1] = {&launch_hm<L1, L2, NT>, &hm_resident<L1, L2, NT>, HmShape<L1, L2, NT>::OS};
     if constexpr (NT < hm_max_nt(L1)) register_hm_nt<L1, L2, NT + 1>(tab);
 }
 
 template <int L1, int L2 = 0>
-static void register_hm_row(HmLaunchFn (*tab)[kMaxPairL + 1][kHmMaxNT])
+static void register_hm_row(HmLaunch (*tab)[kMaxPairL + 1][kHmMaxNT])
 {
     register_hm_nt<L1, L2>(tab);
     if constexpr (L2 < kMaxPairL) register_hm_row<L1, L2 + 1>(tab);
 }
 
-void register_hm_0(HmLaunchFn (*tab)[kMaxPairL + 1][kHmMaxNT]);
-void register_hm_1(HmLaunchFn (*tab)[kMaxPairL + 1][kHmMaxNT]);
-void register_hm_2(HmLaunchFn (*tab)[kMaxPairL + 1][kHmMaxNT]);
-void register_hm_3(HmLaunchFn (*tab)[kMaxPairL + 1][kHmMaxNT]);
-void register_hm_4(HmLaunchFn (*tab)[kMaxPairL + 1][kHmMaxNT]);
-void register_hm_5(HmLaunchFn (*tab)[kMaxPairL + 1][kHmMaxNT]);
-void register_hm_6(HmLaunchFn (*tab)[kMaxPairL + 1][kHmMaxNT]);
+void register_hm_0(HmLaunch (*tab)[kMaxPairL + 1][kHmMaxNT]);
+void register_hm_1(HmLaunch (*tab)[kMaxPairL + 1][kHmMaxNT]);
+void register_hm_2(HmLaunch (*tab)[kMaxPairL + 1][kHmMaxNT]);
+void register_hm_3(HmLaunch (*tab)[kMaxPairL + 1][kHmMaxNT]);
+void register_hm_4(HmLaunch (*tab)[kMaxPairL + 1][kHmMaxNT]);
+void register_hm_5(HmLaunch (*tab)[kMaxPairL + 1][kHmMaxNT]);
+void register_hm_6(HmLaunch (*tab)[kMaxPairL + 1][kHmMaxNT]);
 
 } // namespace gci

@@ -2,5 +2,5 @@
 #include "eri_hermite.cuh"
 
 namespace gci {
-void register_hm_0(HmLaunchFn (*tab)[kMaxPairL + 1][kHmMaxNT]) { register_hm_row<0>(tab); }
+void register_hm_0(HmLaunch (*tab)[kMaxPairL + 1][kHmMaxNT]) { register_hm_row<0>(tab); }
 } // namespace gci

@@ -2,5 +2,5 @@
 #include "eri_hermite.cuh"
 
 namespace gci {
-void register_hm_1(HmLaunchFn (*tab)[kMaxPairL + 1][kHmMaxNT]) { register_hm_row<1>(tab); }
+void register_hm_1(HmLaunch (*tab)[kMaxPairL + 1][kHmMaxNT]) { register_hm_row<1>(tab); }
 } // namespace gci

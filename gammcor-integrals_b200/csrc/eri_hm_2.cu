@@ -2,5 +2,5 @@
 #include "eri_hermite.cuh"
 
 namespace gci {
-void register_hm_2(HmLaunchFn (*tab)[kMaxPairL + 1][kHmMaxNT]) { register_hm_row<2>(tab); }
+void register_hm_2(HmLaunch (*tab)[kMaxPairL + 1][kHmMaxNT]) { register_hm_row<2>(tab); }
 } // namespace gci

@@ -2,5 +2,5 @@
 #include "eri_hermite.cuh"
 
 namespace gci {
-void register_hm_3(HmLaunchFn (*tab)[kMaxPairL + 1][kHmMaxNT]) { register_hm_row<3>(tab); }
+void register_hm_3(HmLaunch (*tab)[kMaxPairL + 1][kHmMaxNT]) { register_hm_row<3>(tab); }
 } // namespace gci

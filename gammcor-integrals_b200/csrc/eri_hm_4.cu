@@ -2,5 +2,5 @@
 #include "eri_hermite.cuh"
 
 namespace gci {
-void register_hm_4(HmLaunchFn (*tab)[kMaxPairL + 1][kHmMaxNT]) { register_hm_row<4>(tab); }
+void register_hm_4(HmLaunch (*tab)[kMaxPairL + 1][kHmMaxNT]) { register_hm_row<4>(tab); }
 } // namespace gci

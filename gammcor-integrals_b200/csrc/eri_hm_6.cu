@@ -2,5 +2,5 @@
 #include "eri_hermite.cuh"
 
 namespace gci {
-void register_hm_6(HmLaunchFn (*tab)[kMaxPairL + 1][kHmMaxNT]) { register_hm_row<6>(tab); }
+void register_hm_6(HmLaunch (*tab)[kMaxPairL + 1][kHmMaxNT]) { register_hm_row<6>(tab); }
 } // namespace gci

@@ -187,26 +187,51 @@ cudaError_t hm_colvec_launch(const HmChunk* chunks, int nchunks, const ShellPair
     return cudaGetLastError();
 }
 
-static HmLaunchFn g_hm[kMaxPairL + 1][kMaxPairL + 1][kHmMaxNT];
+static HmLaunch g_hm[kMaxPairL + 1][kMaxPairL + 1][kHmMaxNT];
 
-static void hm_register()
+static const HmLaunch* hm_class(int L1, int L2, int nt)
 {
-    register_hm_0(g_hm);
-    register_hm_1(g_hm);
-    register_hm_2(g_hm);
-    register_hm_3(g_hm);
-    register_hm_4(g_hm);
-    register_hm_5(g_hm);
-    register_hm_6(g_hm);
+    static std::once_flag once;
+    std::call_once(once, [] {
+        register_hm_0(g_hm);
+        register_hm_1(g_hm);
+        register_hm_2(g_hm);
+        register_hm_3(g_hm);
+        register_hm_4(g_hm);
+        register_hm_5(g_hm);
+        register_hm_6(g_hm);
+    });
+    if (L1 < 0 || L2 < 0 || L1 > kMaxPairL || L2 > kMaxPairL || nt < 1 || nt > hm_max_nt(L1)) return nullptr;
+    const HmLaunch* h = &g_hm[L1][L2][nt - 1];
+    return h->launch ? h : nullptr;
+}
+
+int hm_split(int L1, int L2, int nt, int64_t ntasks, int nib, int nkg, int64_t& doubles)
+{
+    const HmLaunch* h = hm_class(L1, L2, nt);
+    doubles = 0;
+    if (!h || ntasks <= 0) return 1;
+    const int64_t want = h->resident();
+    if (ntasks >= want) return 1;
+    // a part's tensor-core products: below about 4000 (64k cycles of one SM quarter) its own start
+    // and the exchange of its block through L2 are no longer small beside them.  Measured, step-1
+    // integrals: 60 AOs with f shells 95 ms in whole tasks, 37 with this rule; parts down to one
+    // block in every launch below three rounds of the resident warps took 140 AOs from 11.9 to
+    // 23.4 ms, parts for four rounds (of at least 8000 products) 360 AOs from 600 to 717 ms.
+    constexpr int64_t kMinProducts = 4000;
+    const int64_t products = (int64_t)nib * nkg * hm_kt(L2) * hm_mt(L1) * nt;
+    int64_t split = std::min<int64_t>((want + ntasks - 1) / ntasks, nib);
+    split = std::min<int64_t>(split, products / kMinProducts);
+    if (split <= 1) return 1;
+    doubles = ntasks * split * h->block;
+    return (int)split;
 }
 
 cudaError_t hm_launch(int L1, int L2, int nt, const HmArgs& a, cudaStream_t st)
 {
-    static std::once_flag once;
-    std::call_once(once, hm_register);
-    if (L1 < 0 || L2 < 0 || L1 > kMaxPairL || L2 > kMaxPairL || nt < 1 || nt > hm_max_nt(L1) || !g_hm[L1][L2][nt - 1])
-        return cudaErrorInvalidValue;
-    cudaError_t e = g_hm[L1][L2][nt - 1](a, st);
+    const HmLaunch* h = hm_class(L1, L2, nt);
+    if (!h) return cudaErrorInvalidValue;
+    const cudaError_t e = h->launch(a, st);
     count_launch();
     return e;
 }

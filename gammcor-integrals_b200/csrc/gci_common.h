@@ -214,6 +214,13 @@ struct HmArgs {
     double kappa;
     const double* boys;
     unsigned long long* counter;   // task counter of the launch, zero at launch
+    int upper;                     // 1: only tasks whose column pair id is not below the row pair id
+    // a task in `split` parts over its row blocks, for launches with too few tasks to fill the
+    // GPU: part s leaves its block of the output at part[(task * split + s) * (block size)]; the
+    // part that arrives last at arrive[task] (zero at launch) adds them up in order
+    int split;
+    double* part;
+    int* arrive;
 };
 
 // ------------------------------------------------------------ adjoint (Coulomb gradient) path

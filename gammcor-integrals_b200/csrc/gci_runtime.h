@@ -29,6 +29,11 @@ cudaError_t hm_colvec_launch(const HmChunk* chunks, int nchunks, const ShellPair
                              const int* colfun, const double* tmat, const int* toff, const int* nfunc, double* vec,
                              cudaStream_t st);
 cudaError_t hm_launch(int L1, int L2, int nt, const HmArgs& a, cudaStream_t st);
+// Parts per task (HmArgs::split) of a launch of `ntasks` tasks whose longest has `nib` row
+// blocks and `nkg` column groups, and the doubles of HmArgs::part it then needs (0 for one part).
+// A task runs in one warp, so a launch with fewer tasks than resident warps leaves warps idle and
+// lasts as long as its longest task.
+int hm_split(int L1, int L2, int nt, int64_t ntasks, int nib, int nkg, int64_t& doubles);
 // Split-precision FP64 GEMM on the int8 tensor cores (ozaki_gemm.cu):
 // C = alpha A B^T + beta C with A(i, l) = A[i ars + l als], B(j, l) = B[j brs + l bls],
 // k <= ozaki_max_k(); `work` holds ozaki_workspace_bytes(m, n, k); `err` is set to 1
@@ -77,6 +82,8 @@ cudaError_t launch_gather_pivrows(const double* Lb, int nb, const int* piv, int 
 cudaError_t launch_tri_inv_lower(const double* L, int n, double* X, cudaStream_t s);
 cudaError_t launch_downdate(double* D, const double* L, int64_t ld, int64_t n, int ncols, cudaStream_t s);
 cudaError_t launch_max(const double* v, int64_t n, double* out, cudaStream_t s);
+// A(i, j) = A(j, i) where rank[i] > rank[j] (n x n, leading dimension ld).
+cudaError_t launch_mirror(double* A, int64_t ld, int64_t n, const int* rank, cudaStream_t s);
 cudaError_t launch_zero_upper(double* A, int64_t n, cudaStream_t s);
 cudaError_t launch_unpack_rkpq(const double* R, int64_t nvecs, const int64_t* pq_col, const int* pq_ao, int64_t npq,
                                int64_t k0, int64_t kc, int64_t nao, double* U, cudaStream_t s);

@@ -36,3 +36,24 @@ def test_blocks_and_groups_match_class_kernels(gpu_lib, nprim, omega):
     tb = gbasis.from_molecule(mol)
     got, ref = _eri_pairs(gpu_lib, tb, omega, True), _eri_pairs(gpu_lib, tb, omega, False)
     assert np.max(np.abs(got - ref)) <= 1e-12 * np.max(np.abs(ref))
+
+
+def test_parts_and_pairs_without_primitives(gpu_lib):
+    """Few long tasks (36 primitive pairs a side), which run in parts that are added up, among
+    them pairs of steep shells on distant atoms that keep no primitive pair and leave no part."""
+    mol = molecules.random_molecule(32, 2, 6.0, (0, 1, 3), (6, 6), (0.1, 5.0))
+    steep = molecules.random_molecule(33, 2, 6.0, (0, 2), (2, 2), (200.0, 2000.0))
+    atoms = np.array([[0.0, 0.0, 0.0], [5.0, 1.0, 0.5]])
+    shells = sorted(mol.shells + steep.shells, key=lambda s: s[0])
+    tb = gbasis.from_molecule(molecules.Molecule(atoms=atoms, shells=shells))
+    got, ref = _eri_pairs(gpu_lib, tb, 0.0, True), _eri_pairs(gpu_lib, tb, 0.0, False)
+    assert np.max(np.abs(got - ref)) <= 1e-12 * np.max(np.abs(ref))
+    # one block of each two pairs is evaluated and mirrored: exactly symmetric (the block of a pair
+    # with itself is evaluated whole)
+    n = [2 * s[1] + 1 for s in shells]
+    sizes = [n[A] * n[B] if A != B else n[A] * (n[A] + 1) // 2 for B in range(len(n)) for A in range(B, len(n))]
+    pair = np.repeat(np.arange(len(sizes)), sizes)
+    other = pair[:, None] != pair[None, :]
+    assert np.array_equal(got[other], got.T[other])
+    # the parts are added in a fixed order: the same bits again
+    assert np.array_equal(got, _eri_pairs(gpu_lib, tb, 0.0, True))
