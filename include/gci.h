@@ -229,8 +229,9 @@ int gci_trsm_rlt(int64_t rows, int64_t w, double *B, int64_t ldb, const double *
  * full-dimension stage, gci_eri_pairs) contract each pair's primitive
  * Hermite coefficients with the normalised solid-harmonic transforms once,
  * and evaluate every primitive quartet as dense FP64 tensor-core products
- * (the columns a stage keeps times the Hankel matrix R(h + g)).  The class
- * kernels above remain for the diagonal stage and Cartesian bases.
+ * (the columns a stage keeps times the Hankel matrix R(h + g)).  So does
+ * gci_eri_pairs_noalloc where the vectors fit its scratch.  The class kernels
+ * above remain for the diagonal stage and Cartesian bases.
  * enable: 1 on, 0 off, 2 on with per-class timing (the class launches then
  * run one after another, each timed with CUDA events), < 0 query only;
  * returns the previous setting.  Process-wide. */

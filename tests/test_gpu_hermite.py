@@ -57,3 +57,20 @@ def test_parts_and_pairs_without_primitives(gpu_lib):
     assert np.array_equal(got[other], got.T[other])
     # the parts are added in a fixed order: the same bits again
     assert np.array_equal(got, _eri_pairs(gpu_lib, tb, 0.0, True))
+
+
+@pytest.mark.parametrize("nprim", [(2, 3), (5, 6)])
+def test_noalloc_on_both_sides_of_its_scratch(gpu_lib, nprim):
+    """The allocation-free ERI matrix: vectors that fit its scratch (Hermite-matrix kernels) and
+    vectors that do not (class kernels), against gci_eri_pairs."""
+    import torch
+    tb = gbasis.from_molecule(molecules.random_molecule(34, 1, 4.0, molecules.RECIPE_C2, nprim, (0.1, 50.0)))
+    npq = tb.NAO * (tb.NAO + 1) // 2
+    out = torch.full((npq, npq + 5), float("nan"), dtype=torch.float64, device="cuda")
+    s = tb.c_struct()
+    stream = torch.cuda.current_stream()
+    _capi.check(gpu_lib.gci_eri_pairs_noalloc(C.byref(s), 0.3, C.c_void_p(out.data_ptr()), npq + 5,
+                                              C.c_void_p(stream.cuda_stream)))
+    got, ref = out.cpu().numpy().T, _eri_pairs(gpu_lib, tb, 0.3, True)
+    assert np.max(np.abs(got[:npq] - ref)) <= 1e-12 * np.max(np.abs(ref))
+    assert np.all(got[npq:] == 0.0)
