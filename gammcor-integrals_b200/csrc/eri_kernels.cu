@@ -21,74 +21,93 @@ __global__ void k_pair_records(const ShellPairDev* __restrict__ pairs, int npair
                                const double* __restrict__ exps, const double* __restrict__ coefs,
                                const int* __restrict__ plist, double* __restrict__ pp)
 {
+    // extents (x | y << 8 | z << 16) and table offsets of the pair's Cartesian pairs, and the
+    // position of their products
+    constexpr int kMaxE = ncart(kMaxL) * ncart(kMaxL);
+    __shared__ int ext[kMaxE], ox[kMaxE], oy[kMaxE], oz[kMaxE], first[kMaxE];
     for (int p = blockIdx.x; p < npairs; p += gridDim.x) {
         const ShellPairDev sp = pairs[p];
         const int la = sp.l1, lb = sp.l2;
-        const int rs = pp_record(la, lb);
-        const int ne = e2_size(la, lb);
+        const int rs = pp_record(la, lb), po = pp_prod_off(la, lb);
+        const int ne = e2_size(la, lb), nE = ncart(la) * ncart(lb);
         const int n = sp.npp;
         const double ax = xyz[3 * sp.s1], ay = xyz[3 * sp.s1 + 1], az = xyz[3 * sp.s1 + 2];
         const double bx = xyz[3 * sp.s2], by = xyz[3 * sp.s2 + 1], bz = xyz[3 * sp.s2 + 2];
         const double r2 = (ax - bx) * (ax - bx) + (ay - by) * (ay - by) + (az - bz) * (az - bz);
-        for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        __syncthreads();   // the previous pair's readers are done
+        for (int e = threadIdx.x; e < nE; e += blockDim.x) {
+            ext[e] = pair_x(la, lb, e) | (pair_y(la, lb, e) << 8) | (pair_z(la, lb, e) << 16);
+            ox[e] = pair_ox(la, lb, e); oy[e] = pair_oy(la, lb, e); oz[e] = pair_oz(la, lb, e);
+        }
+        // one thread per primitive pair and axis: the table of that axis
+        for (int w = threadIdx.x; w < 3 * n; w += blockDim.x) {
+            const int i = w / 3, axis = w - 3 * i;
             const int code = plist[sp.list_off + i];
             const int ga = code & 0xff, gb = code >> 8;
             const double ea = exps[poff[sp.s1] + ga], eb = exps[poff[sp.s2] + gb];
-            const double ca = coefs[poff[sp.s1] + ga], cb = coefs[poff[sp.s2] + gb];
             const double P = ea + eb;
-            const double px = (ea * ax + eb * bx) / P, py = (ea * ay + eb * by) / P, pz = (ea * az + eb * bz) / P;
+            const double A = axis == 0 ? ax : (axis == 1 ? ay : az), B = axis == 0 ? bx : (axis == 1 ? by : bz);
+            const double pc = (ea * A + eb * B) / P, PA = pc - A, PB = pc - B;
             double* rec = pp + sp.rec_off + (size_t)i * rs;
-            rec[0] = P; rec[1] = px; rec[2] = py; rec[3] = pz;
-            rec[4] = exp(-ea * eb / P * r2) * ca * cb;
-            rec[5] = px - ax; rec[6] = py - ay; rec[7] = pz - az;
+            rec[1 + axis] = pc;
+            rec[5 + axis] = PA;
+            if (axis == 0) {
+                rec[0] = P;
+                rec[4] = exp(-ea * eb / P * r2) * coefs[poff[sp.s1] + ga] * coefs[poff[sp.s2] + gb];
+            }
             const double h = 1.0 / (2.0 * P);
-            const double PA[3] = {px - ax, py - ay, pz - az};
-            const double PB[3] = {px - bx, py - by, pz - bz};
-            for (int axis = 0; axis < 3; ++axis) {
-                double* E = rec + 8 + axis * ne;
-                E[0] = 1.0;
-                // raise i on A: E^{i+1,0}
-                for (int a = 0; a < la; ++a) {
-                    const double* Ei = E + e2_off(la, a, 0);
-                    double* En = E + e2_off(la, a + 1, 0);
-                    for (int t = 0; t <= a + 1; ++t) {
+            double* E = rec + 8 + axis * ne;
+            E[0] = 1.0;
+            // raise i on A: E^{i+1,0}
+            for (int a = 0; a < la; ++a) {
+                const double* Ei = E + e2_off(la, a, 0);
+                double* En = E + e2_off(la, a + 1, 0);
+                for (int t = 0; t <= a + 1; ++t) {
+                    double v = 0.0;
+                    if (t >= 1) v += h * Ei[t - 1];
+                    if (t <= a) v += PA * Ei[t];
+                    if (t + 1 <= a) v += (double)(t + 1) * Ei[t + 1];
+                    En[t] = v;
+                }
+            }
+            // raise j on B: E^{i,j+1}
+            for (int b = 0; b < lb; ++b)
+                for (int a = 0; a <= la; ++a) {
+                    const double* Ej = E + e2_off(la, a, b);
+                    double* En = E + e2_off(la, a, b + 1);
+                    const int m = a + b;
+                    for (int t = 0; t <= m + 1; ++t) {
                         double v = 0.0;
-                        if (t >= 1) v += h * Ei[t - 1];
-                        if (t <= a) v += PA[axis] * Ei[t];
-                        if (t + 1 <= a) v += (double)(t + 1) * Ei[t + 1];
+                        if (t >= 1) v += h * Ej[t - 1];
+                        if (t <= m) v += PB * Ej[t];
+                        if (t + 1 <= m) v += (double)(t + 1) * Ej[t + 1];
                         En[t] = v;
                     }
                 }
-                // raise j on B: E^{i,j+1}
-                for (int b = 0; b < lb; ++b)
-                    for (int a = 0; a <= la; ++a) {
-                        const double* Ej = E + e2_off(la, a, b);
-                        double* En = E + e2_off(la, a, b + 1);
-                        const int m = a + b;
-                        for (int t = 0; t <= m + 1; ++t) {
-                            double v = 0.0;
-                            if (t >= 1) v += h * Ej[t - 1];
-                            if (t <= m) v += PB[axis] * Ej[t];
-                            if (t + 1 <= m) v += (double)(t + 1) * Ej[t + 1];
-                            En[t] = v;
-                        }
-                    }
-            }
-            // Hermite products of every Cartesian pair (b fastest), v outer, t inner
-            const double* Ex = rec + 8;
-            const double* Ey = Ex + ne;
-            const double* Ez = Ey + ne;
-            double* prod = rec + pp_prod_off(la, lb);
+        }
+        __syncthreads();
+        for (int e = threadIdx.x; e < nE; e += blockDim.x) {
             int c = 0;
-            for (int e = 0; e < ncart(la) * ncart(lb); ++e) {
-                const int ex = pair_x(la, lb, e), ey = pair_y(la, lb, e), ez = pair_z(la, lb, e);
-                const int ox = pair_ox(la, lb, e), oy = pair_oy(la, lb, e), oz = pair_oz(la, lb, e);
-                for (int v = 0; v <= ez; ++v)
-                    for (int u = 0; u <= ey; ++u) {
-                        const double yz = Ey[oy + u] * Ez[oz + v];
-                        for (int t = 0; t <= ex; ++t) prod[c++] = Ex[ox + t] * yz;
-                    }
-            }
+            for (int f = 0; f < e; ++f) c += ((ext[f] & 255) + 1) * (((ext[f] >> 8) & 255) + 1) * ((ext[f] >> 16) + 1);
+            first[e] = c;
+        }
+        __syncthreads();
+        // one thread per primitive pair and Cartesian pair (b fastest): its Hermite products, v
+        // outer, t inner
+        for (int w = threadIdx.x; w < n * nE; w += blockDim.x) {
+            const int i = w / nE, e = w - i * nE;
+            double* rec = pp + sp.rec_off + (size_t)i * rs;
+            const double* Ex = rec + 8 + ox[e];
+            const double* Ey = rec + 8 + ne + oy[e];
+            const double* Ez = rec + 8 + 2 * ne + oz[e];
+            double* prod = rec + po + first[e];
+            const int ex = ext[e] & 255, ey = (ext[e] >> 8) & 255, ez = ext[e] >> 16;
+            int c = 0;
+            for (int v = 0; v <= ez; ++v)
+                for (int u = 0; u <= ey; ++u) {
+                    const double yz = Ey[u] * Ez[v];
+                    for (int t = 0; t <= ex; ++t) prod[c++] = Ex[t] * yz;
+                }
         }
     }
 }

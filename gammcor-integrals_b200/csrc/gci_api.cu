@@ -1860,7 +1860,10 @@ static void coulomb_grad_impl(const gci_basis* basis, double omega, const double
                                 db.exps.p, db.coefs.p, P.plist.p, db.tmat.p, db.toff.p, db.nfunc.p, db.loc.p, Dp, ldd,
                                 mP.p, mX.p, mY.p, mZ.p, vecs.p, hk.p, d_ppair.p, C.stream));
     CU(cudaMemsetAsync(V.p, 0, sizeof(double) * V.n, C.stream));
-    constexpr int64_t kChunk = 512;   // ket primitive pairs per warp
+    // the classes only share the potentials, which they add to atomically: spread over the
+    // auxiliary streams, so that the short ones of a small molecule overlap
+    fork_streams(C);
+    int li = 0;
     for (int L1 = 0; L1 < NL; ++L1)
         for (int L2 = 0; L2 < NL; ++L2) {
             g_grad_work[L1][L2] = (double)ln[L1] * (double)ln[L2];
@@ -1871,12 +1874,16 @@ static void coulomb_grad_impl(const gci_basis* basis, double omega, const double
             a.ket_beg = lbeg[L2]; a.nket = ln[L2];
             a.hk = hk.p + hk_off[L2];
             a.V = V.p + pot_off[L1];
-            a.chunk = kChunk;
-            a.nchunk = (ln[L2] + kChunk - 1) / kChunk;
+            // ket primitive pairs per warp: 512, which leaves the warp's final sum over its lanes
+            // below a tenth of its work, less where that gives fewer than 16 warps an SM
+            a.chunk = 512;
+            while (a.chunk > 64 && a.nbra * ((a.nket + a.chunk - 1) / a.chunk) < 148 * 16) a.chunk /= 2;
+            a.nchunk = (a.nket + a.chunk - 1) / a.chunk;
             a.kappa = H.kappa;
             a.boys = g_ctx.boys.p;
-            CU(grad_potential_launch(L1, L2, a, C.stream));
+            CU(grad_potential_launch(L1, L2, a, C.aux[li++ % kAuxStreams]));
         }
+    join_streams(C);
     for (int L = 0; L < NL; ++L)
         CU(grad_dots_launch(lbeg[L], ln[L], grad_hb(L), vecs.p + vec_off[L], V.p + pot_off[L], dots.p, C.stream));
     if (jmat) {

@@ -16,11 +16,9 @@ struct GradE {
     double e[NI][NI][NT];
 };
 
+// Fills a table that is zero on entry.
 __device__ static void grad_etab(GradE& E, int la, int lb, double PA, double PB, double h)
 {
-    for (int i = 0; i < GradE::NI; ++i)
-        for (int j = 0; j < GradE::NI; ++j)
-            for (int t = 0; t < GradE::NT; ++t) E.e[i][j][t] = 0.0;
     E.e[0][0][0] = 1.0;
     for (int i = 0; i <= la; ++i)
         for (int t = 0; t <= i + 1; ++t) {
@@ -41,9 +39,14 @@ __device__ static void grad_etab(GradE& E, int la, int lb, double PA, double PB,
 
 // One block per shell pair: the Cartesian density block Ds (symmetrised,
 // times w_AB, with the norms and spherical transforms of both shells) in
-// shared memory, then one thread per kept primitive pair writes its seven
+// shared memory, then one warp per kept primitive pair writes its seven
 // Hermite vectors (h, gA, gB; grad_hb(L) entries each), its geometry and,
-// transposed and signed, its ket vector.
+// transposed and signed, its ket vector: three lanes fill the axes' tables in
+// shared memory, then each lane sums whole entries over the Cartesian pairs in
+// registers.  (One thread per primitive pair, with its tables in local memory
+// and its entries accumulated in global memory, is a chain of thousands of
+// dependent accesses.)  80 us on 42 AOs, latency of the tables' recursion.
+constexpr int kGradVecWarps = 2;
 __global__ void k_grad_pair_vectors(const ShellPairDev* __restrict__ pairs, int npairs,
                                     const int64_t* __restrict__ gbase, const int* __restrict__ level_beg,
                                     const int* __restrict__ level_n, const int64_t* __restrict__ vec_off,
@@ -57,6 +60,15 @@ __global__ void k_grad_pair_vectors(const ShellPairDev* __restrict__ pairs, int 
                                     double* __restrict__ vecs, double* __restrict__ hk, int* __restrict__ ppair)
 {
     __shared__ double Dc[ncart(kMaxL) * ncart(kMaxL)];
+    __shared__ int cart[2][ncart(kMaxL)];            // x | y << 8 | z << 16 of the components of both shells
+    __shared__ int herm[grad_hb(2 * kMaxL)];         // t | u << 8 | v << 16
+    __shared__ GradE tabs[kGradVecWarps][3];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    GradE& Ex = tabs[warp][0];
+    GradE& Ey = tabs[warp][1];
+    GradE& Ez = tabs[warp][2];
+    for (int h = threadIdx.x; h < grad_hb(2 * kMaxL); h += blockDim.x)
+        herm[h] = herm_t(h) | (herm_u(h) << 8) | (herm_v(h) << 16);
     for (int p = blockIdx.x; p < npairs; p += gridDim.x) {
         const ShellPairDev sp = pairs[p];
         const int s1 = sp.s1, s2 = sp.s2, la = sp.l1, lb = sp.l2, L = la + lb;
@@ -79,13 +91,18 @@ __global__ void k_grad_pair_vectors(const ShellPairDev* __restrict__ pairs, int 
             }
             Dc[e] = w * acc;
         }
+        if (threadIdx.x < nc1 + nc2) {
+            const int which = threadIdx.x >= nc1, c = which ? threadIdx.x - nc1 : threadIdx.x;
+            const int g = cart_off(which ? lb : la) + c;
+            cart[which][c] = cart_x(g) | (cart_y(g) << 8) | (cart_z(g) << 16);
+        }
         __syncthreads();
         const double ax = xyz[3 * s1], ay = xyz[3 * s1 + 1], az = xyz[3 * s1 + 2];
         const double bx = xyz[3 * s2], by = xyz[3 * s2 + 1], bz = xyz[3 * s2 + 2];
         const double r2 = (ax - bx) * (ax - bx) + (ay - by) * (ay - by) + (az - bz) * (az - bz);
         const int HB = grad_hb(L);
         const int HL = herm_n(L);
-        for (int i = threadIdx.x; i < sp.npp; i += blockDim.x) {
+        for (int i = warp; i < sp.npp; i += kGradVecWarps) {
             const int code = plist[sp.list_off + i];
             const int ga = code & 0xff, gb = code >> 8;
             const double ea = exps[poff[s1] + ga], eb = exps[poff[s2] + gb];
@@ -94,84 +111,96 @@ __global__ void k_grad_pair_vectors(const ShellPairDev* __restrict__ pairs, int 
             const double px = (ea * ax + eb * bx) / P, py = (ea * ay + eb * by) / P, pz = (ea * az + eb * bz) / P;
             const double K = exp(-ea * eb / P * r2) * ca * cb;
             const double h = 1.0 / (2.0 * P);
-            GradE Ex, Ey, Ez;
-            grad_etab(Ex, la, lb, px - ax, px - bx, h);
-            grad_etab(Ey, la, lb, py - ay, py - by, h);
-            grad_etab(Ez, la, lb, pz - az, pz - bz, h);
+            __syncwarp();   // the previous primitive pair's readers are done
+            double* tz = &tabs[warp][0].e[0][0][0];
+            for (int e = lane; e < 3 * GradE::NI * GradE::NI * GradE::NT; e += 32) tz[e] = 0.0;
+            __syncwarp();
+            if (lane < 3) {
+                const double pc = lane == 0 ? px : (lane == 1 ? py : pz);
+                const double ac = lane == 0 ? ax : (lane == 1 ? ay : az), bc = lane == 0 ? bx : (lane == 1 ? by : bz);
+                grad_etab(tabs[warp][lane], la, lb, pc - ac, pc - bc, h);
+            }
+            __syncwarp();
             const int64_t g = gbase[p] + i;
             const int64_t li = g - level_beg[L];
+            const int64_t nL = level_n[L];
             double* vg = vecs + vec_off[L] + li * (int64_t)(kGradVec * HB);
-            for (int c = 0; c < kGradVec * HB; ++c) vg[c] = 0.0;
-            for (int a = 0; a < nc1; ++a) {
-                const int A = cart_off(la) + a;
-                const int axx = cart_x(A), ayy = cart_y(A), azz = cart_z(A);
-                for (int b = 0; b < nc2; ++b) {
-                    const double d = K * Dc[a * nc2 + b];
-                    if (d == 0.0) continue;
-                    const int B = cart_off(lb) + b;
-                    const int bxx = cart_x(B), byy = cart_y(B), bzz = cart_z(B);
-                    // (t, u, v) up to one unit above the pair's range on each axis, but
-                    // only up to level L + 1 in total: every nonzero product lies there,
-                    // and the vector block of this primitive pair ends there
-                    for (int v = 0; v <= azz + bzz + 1; ++v) {
+            // entry (t, u, v) of the seven vectors: every nonzero product lies within one unit above
+            // the pair's range on each axis, and within level L + 1 in total
+            for (int hh = lane; hh < HB; hh += 32) {
+                const int t = herm[hh] & 255, u = (herm[hh] >> 8) & 255, v = herm[hh] >> 16;
+                double s[kGradVec] = {};
+                for (int a = 0; a < nc1; ++a) {
+                    const int A = cart[0][a], axx = A & 255, ayy = (A >> 8) & 255, azz = A >> 16;
+                    for (int b = 0; b < nc2; ++b) {
+                        const double d = K * Dc[a * nc2 + b];
+                        const int B = cart[1][b], bxx = B & 255, byy = (B >> 8) & 255, bzz = B >> 16;
+                        if (d == 0.0 || t > axx + bxx + 1 || u > ayy + byy + 1 || v > azz + bzz + 1) continue;
                         const double z0 = Ez.e[azz][bzz][v];
                         const double zA = 2.0 * ea * Ez.e[azz + 1][bzz][v] - (azz > 0 ? azz * Ez.e[azz - 1][bzz][v] : 0.0);
                         const double zB = 2.0 * eb * Ez.e[azz][bzz + 1][v] - (bzz > 0 ? bzz * Ez.e[azz][bzz - 1][v] : 0.0);
-                        for (int u = 0; u <= ayy + byy + 1 && u + v <= L + 1; ++u) {
-                            const double y0 = Ey.e[ayy][byy][u];
-                            const double yA = 2.0 * ea * Ey.e[ayy + 1][byy][u] - (ayy > 0 ? ayy * Ey.e[ayy - 1][byy][u] : 0.0);
-                            const double yB = 2.0 * eb * Ey.e[ayy][byy + 1][u] - (byy > 0 ? byy * Ey.e[ayy][byy - 1][u] : 0.0);
-                            for (int t = 0; t <= axx + bxx + 1 && t + u + v <= L + 1; ++t) {
-                                const double x0 = Ex.e[axx][bxx][t];
-                                const double xA = 2.0 * ea * Ex.e[axx + 1][bxx][t] - (axx > 0 ? axx * Ex.e[axx - 1][bxx][t] : 0.0);
-                                const double xB = 2.0 * eb * Ex.e[axx][bxx + 1][t] - (bxx > 0 ? bxx * Ex.e[axx][bxx - 1][t] : 0.0);
-                                const int hh = herm_idx(t, u, v);
-                                vg[0 * HB + hh] += d * x0 * y0 * z0;
-                                vg[1 * HB + hh] += d * xA * y0 * z0;
-                                vg[2 * HB + hh] += d * x0 * yA * z0;
-                                vg[3 * HB + hh] += d * x0 * y0 * zA;
-                                vg[4 * HB + hh] += d * xB * y0 * z0;
-                                vg[5 * HB + hh] += d * x0 * yB * z0;
-                                vg[6 * HB + hh] += d * x0 * y0 * zB;
-                            }
-                        }
+                        const double y0 = Ey.e[ayy][byy][u];
+                        const double yA = 2.0 * ea * Ey.e[ayy + 1][byy][u] - (ayy > 0 ? ayy * Ey.e[ayy - 1][byy][u] : 0.0);
+                        const double yB = 2.0 * eb * Ey.e[ayy][byy + 1][u] - (byy > 0 ? byy * Ey.e[ayy][byy - 1][u] : 0.0);
+                        const double x0 = Ex.e[axx][bxx][t];
+                        const double xA = 2.0 * ea * Ex.e[axx + 1][bxx][t] - (axx > 0 ? axx * Ex.e[axx - 1][bxx][t] : 0.0);
+                        const double xB = 2.0 * eb * Ex.e[axx][bxx + 1][t] - (bxx > 0 ? bxx * Ex.e[axx][bxx - 1][t] : 0.0);
+                        s[0] += d * x0 * y0 * z0;
+                        s[1] += d * xA * y0 * z0;
+                        s[2] += d * x0 * yA * z0;
+                        s[3] += d * x0 * y0 * zA;
+                        s[4] += d * xB * y0 * z0;
+                        s[5] += d * x0 * yB * z0;
+                        s[6] += d * x0 * y0 * zB;
                     }
                 }
+#pragma unroll
+                for (int c = 0; c < kGradVec; ++c) vg[c * HB + hh] = s[c];
+                // ket role: (-1)^{tau+nu+phi} h(tau), transposed within the level
+                if (hh < HL) hk[hk_off[L] + (int64_t)hh * nL + li] = ((t + u + v) & 1) ? -s[0] : s[0];
             }
-            mP[g] = P; mX[g] = px; mY[g] = py; mZ[g] = pz;
-            ppair[g] = p;
-            // ket role: (-1)^{tau+nu+phi} h(tau), transposed within the level
-            const int64_t nL = level_n[L];
-            for (int tau = 0; tau < HL; ++tau) {
-                const int s = herm_level(tau);
-                hk[hk_off[L] + (int64_t)tau * nL + li] = (s & 1) ? -vg[tau] : vg[tau];
+            if (lane == 0) {
+                mP[g] = P; mX[g] = px; mY[g] = py; mZ[g] = pz;
+                ppair[g] = p;
             }
         }
     }
 }
 
-// One thread per primitive pair: the seven dot products of its vectors with
-// its potential, out[g * 7 + c] (c = 0: h.V, 1..3: gA.V, 4..6: gB.V).
+// One warp per primitive pair: the seven dot products of its vectors with its
+// potential, out[g * 7 + c] (c = 0: h.V, 1..3: gA.V, 4..6: gB.V); the lanes read
+// consecutive entries (one read of the vectors: bound by HBM).
 __global__ void k_grad_dots(int64_t beg, int64_t n, int HB, const double* __restrict__ vecs,
                             const double* __restrict__ V, double* __restrict__ out)
 {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const int lane = threadIdx.x & 31;
+    const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+    for (int64_t i = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < n; i += warps) {
         const double* vg = vecs + i * (int64_t)(kGradVec * HB);
         const double* vi = V + i * (int64_t)HB;
+        double s[kGradVec] = {};
+        for (int h = lane; h < HB; h += 32) {
+            const double v = vi[h];
+#pragma unroll
+            for (int c = 0; c < kGradVec; ++c) s[c] = fma(vg[c * HB + h], v, s[c]);
+        }
+#pragma unroll
         for (int c = 0; c < kGradVec; ++c) {
-            double s = 0.0;
-            for (int h = 0; h < HB; ++h) s += vg[c * HB + h] * vi[h];
-            out[(beg + i) * kGradVec + c] = s;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) s[c] += __shfl_xor_sync(0xffffffffu, s[c], o);
+            if (lane == c) out[(beg + i) * kGradVec + c] = s[c];
         }
     }
 }
 
 // Coulomb matrix J_pq = sum_rs (pq|rs) Ds_rs: one block per shell pair; a
-// thread per Cartesian pair (a, b) contracts the pair's primitive-pair
+// few threads per Cartesian pair (a, b) contract the pair's primitive-pair
 // records (K c_a c_b and the Hermite products E^{ab}_tuv, as the ERI kernels
-// read them) with the potentials, then the block applies the two shells'
-// transforms and writes the (s1, s2) block and its transpose.
-__global__ void k_grad_coulomb_matrix(const ShellPairDev* __restrict__ pairs, int npairs,
+// read them) with the potentials, each every few primitive pairs, then the
+// block applies the two shells' transforms and writes the (s1, s2) block and its
+// transpose.
+constexpr int kGradMatThreads = 256;
+__global__ void __launch_bounds__(kGradMatThreads) k_grad_coulomb_matrix(const ShellPairDev* __restrict__ pairs, int npairs,
                                       const int64_t* __restrict__ gbase, const int* __restrict__ level_beg,
                                       const int64_t* __restrict__ pot_off, const double* __restrict__ V,
                                       const double* __restrict__ pp, const double* __restrict__ tmat,
@@ -179,7 +208,9 @@ __global__ void k_grad_coulomb_matrix(const ShellPairDev* __restrict__ pairs, in
                                       const int* __restrict__ loc, double* __restrict__ J, int64_t ldj)
 {
     __shared__ double Jc[ncart(kMaxL) * ncart(kMaxL)];
-    __shared__ double Jh[(2 * kMaxL + 1) * ncart(kMaxL)];
+    __shared__ double Jh[ncart(kMaxL) * ncart(kMaxL)];
+    __shared__ int ext[ncart(kMaxL) * ncart(kMaxL)];   // Hermite extent of every Cartesian pair
+    __shared__ double part[kGradMatThreads];
     for (int p = blockIdx.x; p < npairs; p += gridDim.x) {
         const ShellPairDev sp = pairs[p];
         const int s1 = sp.s1, s2 = sp.s2, la = sp.l1, lb = sp.l2, L = la + lb;
@@ -187,12 +218,16 @@ __global__ void k_grad_coulomb_matrix(const ShellPairDev* __restrict__ pairs, in
         const int HB = grad_hb(L);
         const int rs = pp_record(la, lb), po = pp_prod_off(la, lb);
         __syncthreads();
-        for (int e = threadIdx.x; e < nc1 * nc2; e += blockDim.x) {
+        for (int e = threadIdx.x; e < nc1 * nc2; e += blockDim.x) ext[e] = pair_x(la, lb, e) | (pair_y(la, lb, e) << 8) | (pair_z(la, lb, e) << 16);
+        __syncthreads();
+        const int nE = nc1 * nc2, per = kGradMatThreads / nE;   // threads per Cartesian pair (nE <= 100)
+        if (threadIdx.x < per * nE) {
+            const int e = threadIdx.x % nE;
             int off = 0;
-            for (int f = 0; f < e; ++f) off += pair_supp(la, lb, f);
-            const int ex = pair_x(la, lb, e), ey = pair_y(la, lb, e), ez = pair_z(la, lb, e);
+            for (int f = 0; f < e; ++f) off += ((ext[f] & 255) + 1) * (((ext[f] >> 8) & 255) + 1) * ((ext[f] >> 16) + 1);
+            const int ex = ext[e] & 255, ey = (ext[e] >> 8) & 255, ez = ext[e] >> 16;
             double acc = 0.0;
-            for (int i = 0; i < sp.npp; ++i) {
+            for (int i = threadIdx.x / nE; i < sp.npp; i += per) {
                 const double* rec = pp + sp.rec_off + (int64_t)i * rs;
                 const double* prod = rec + po + off;
                 const int64_t g = gbase[p] + i;
@@ -204,6 +239,12 @@ __global__ void k_grad_coulomb_matrix(const ShellPairDev* __restrict__ pairs, in
                         for (int t = 0; t <= ex; ++t) s += prod[c++] * vi[herm_idx(t, u, v)];
                 acc += rec[4] * s;
             }
+            part[threadIdx.x] = acc;
+        }
+        __syncthreads();
+        for (int e = threadIdx.x; e < nE; e += blockDim.x) {
+            double acc = 0.0;
+            for (int q = 0; q < per; ++q) acc += part[q * nE + e];
             Jc[e] = acc;
         }
         __syncthreads();
@@ -251,7 +292,7 @@ cudaError_t grad_pair_vectors_launch(const ShellPairDev* pairs, int npairs, cons
 {
     if (npairs <= 0) return cudaSuccess;
     const int blocks = npairs < 148 * 32 ? npairs : 148 * 32;
-    k_grad_pair_vectors<<<blocks, 64, 0, st>>>(pairs, npairs, gbase, level_beg, level_n, vec_off, hk_off, xyz, poff,
+    k_grad_pair_vectors<<<blocks, 32 * kGradVecWarps, 0, st>>>(pairs, npairs, gbase, level_beg, level_n, vec_off, hk_off, xyz, poff,
                                                exps, coefs, plist, tmat, toff, nfunc, loc, D, ldd, mP, mX, mY, mZ,
                                                vecs, hk, ppair);
     count_launch();
@@ -271,7 +312,7 @@ cudaError_t grad_dots_launch(int64_t beg, int64_t n, int HB, const double* vecs,
                              cudaStream_t st)
 {
     if (n <= 0) return cudaSuccess;
-    int64_t blocks = (n + 127) / 128;
+    int64_t blocks = (n + 3) / 4;
     if (blocks > 148 * 16) blocks = 148 * 16;
     k_grad_dots<<<(unsigned)blocks, 128, 0, st>>>(beg, n, HB, vecs, V, out);
     count_launch();
@@ -285,7 +326,7 @@ cudaError_t grad_coulomb_matrix_launch(const ShellPairDev* pairs, int npairs, co
 {
     if (npairs <= 0) return cudaSuccess;
     const int blocks = npairs < 148 * 32 ? npairs : 148 * 32;
-    k_grad_coulomb_matrix<<<blocks, 128, 0, st>>>(pairs, npairs, gbase, level_beg, pot_off, V, pp, tmat, toff, nfunc,
+    k_grad_coulomb_matrix<<<blocks, kGradMatThreads, 0, st>>>(pairs, npairs, gbase, level_beg, pot_off, V, pp, tmat, toff, nfunc,
                                                   loc, J, ldj);
     count_launch();
     return cudaGetLastError();
