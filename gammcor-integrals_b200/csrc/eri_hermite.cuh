@@ -192,12 +192,9 @@ __device__ __noinline__ void hm_produce(const double* __restrict__ Bp, const dou
 {
     const double P = __ldg(Bp), Q = __ldg(Kp);
     const double dx = __ldg(Bp + 1) - __ldg(Kp + 1), dy = __ldg(Bp + 2) - __ldg(Kp + 2), dz = __ldg(Bp + 3) - __ldg(Kp + 3);
-    // Boys values scaled by 2 pi^{5/2} / (PQ sqrt(P+Q+kappa PQ)) (auto2e_WMatrix_part1.f90:134)
-    // and (-2 alpha)^m
-    const double PQ = P * Q;
-    const double den = P + Q + kappa * PQ;
-    const double alpha = PQ / den;
-    const double pref = 34.986836655249725 / (PQ * sqrt(den));
+    // Boys values scaled by the quartet's factor and (-2 alpha)^m
+    double alpha, pref;
+    quartet_factors(P, Q, kappa, alpha, pref);
     double F[LT + 1];
     boys_fm<LT>(alpha * (dx * dx + dy * dy + dz * dz), boys, F);
     double pw = on ? pref : 0.0;

@@ -2515,7 +2515,7 @@ int gci_eri_pairs_noalloc(const gci_basis* basis, double omega, double* out_dev,
             std::vector<int64_t> pos(seg.begin(), seg.end() - 1);
             for (int64_t sp = 0; sp < P.n; ++sp) ids[pos[P.type[sp]]++] = (int)sp;
         }
-        // the table of the Boys function depends on nothing but its order: computed once (9 ms)
+        // the table of the Boys function depends on nothing but its order: computed once (8 ms)
         static const std::vector<double> boys = boys_table(kBoysMaxM);
 
         // scratch layout; reject before touching the device if it does not fit
@@ -2533,7 +2533,7 @@ int gci_eri_pairs_noalloc(const gci_basis* basis, double omega, double* out_dev,
                                      std::to_string(kNoAllocScratchBytes) + " (use gci_eri_pairs for this basis)");
 
         // spherical bases run on the Hermite-matrix kernels where their vectors fit the rest of the
-        // scratch too (42 AOs: 3.0 ms against 6 on the class kernels, whose launches are each as long as
+        // scratch too (42 AOs: 3.0 ms against 7.7 on the class kernels, whose launches are each as long as
         // their longest quartet), else on the class kernels
         bool hm = g_hm_enabled.load() && hb.spher;
         std::vector<int64_t> rowoff(P.n, 0);

@@ -85,9 +85,8 @@ __global__ void __launch_bounds__(128) k_grad_potential(const GradPotArgs a)
         const int64_t gk = a.ket_beg + k;
         const double Q = __ldg(a.mP + gk);
         const double X = px - __ldg(a.mX + gk), Y = py - __ldg(a.mY + gk), Z = pz - __ldg(a.mZ + gk);
-        const double PQ = P * Q, den = P + Q + a.kappa * PQ;
-        const double alpha = PQ / den;
-        const double pref = 2.0 * 17.49341832762486284626282167987155377876 / (PQ * sqrt(den));   // 2 pi^{5/2}
+        double alpha, pref;
+        quartet_factors(P, Q, a.kappa, alpha, pref);
         double F[N + 1];
         boys_fm<N>(alpha * (X * X + Y * Y + Z * Z), a.boys, F);
         double Fs[N + 1];
