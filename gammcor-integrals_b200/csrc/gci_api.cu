@@ -133,7 +133,7 @@ struct Context {
     int device = 0;
     cudaStream_t stream = nullptr;
     // streams on which independent class launches of one ERI stage overlap
-    // (forked from and joined back into `stream` by events), created on first use
+    // (forked from and joined back into `stream` by events)
     cudaStream_t aux[kAuxStreams] = {};
     cudaEvent_t ev_fork = nullptr;
     cudaEvent_t ev_join[kAuxStreams] = {};
@@ -151,6 +151,11 @@ static void context_streams(Context& c)
 {
     CU(cudaGetDevice(&c.device));
     CU(cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking));
+    CU(cudaEventCreateWithFlags(&c.ev_fork, cudaEventDisableTiming));
+    for (int q = 0; q < kAuxStreams; ++q) {
+        CU(cudaStreamCreateWithFlags(&c.aux[q], cudaStreamNonBlocking));
+        CU(cudaEventCreateWithFlags(&c.ev_join[q], cudaEventDisableTiming));
+    }
 }
 
 static Context& ctx()
@@ -554,16 +559,10 @@ static void hm_ensure_rows(Handle& H, const std::vector<int>& ids)
     for (int64_t id = 0; id < P.n; ++id) H.hm_rowoff_h[id] = want[id] ? off[id] : -1;
 }
 
-// Auxiliary streams of the context, forked from its stream (C.ev_fork recorded) / joined back.
+// Auxiliary streams of the context, forked from its stream / joined back.  Threads that share a
+// context may interleave: a wait then takes the other thread's later record on the same stream.
 static void fork_streams(Context& C)
 {
-    if (!C.ev_fork) {
-        CU(cudaEventCreateWithFlags(&C.ev_fork, cudaEventDisableTiming));
-        for (int q = 0; q < kAuxStreams; ++q) {
-            CU(cudaStreamCreateWithFlags(&C.aux[q], cudaStreamNonBlocking));
-            CU(cudaEventCreateWithFlags(&C.ev_join[q], cudaEventDisableTiming));
-        }
-    }
     CU(cudaEventRecord(C.ev_fork, C.stream));
     for (int q = 0; q < kAuxStreams; ++q) CU(cudaStreamWaitEvent(C.aux[q], C.ev_fork, 0));
 }
