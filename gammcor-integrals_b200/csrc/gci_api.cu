@@ -1784,6 +1784,8 @@ struct gci_handle {
 // ------------------------------------------------------------------ adjoint: Coulomb energy and gradient
 // Work of the last gci_coulomb_grad call: primitive quartets per (bra level, ket level).
 static double g_grad_work[kGradMaxL + 1][kGradMaxL + 1];
+// Entries of the chunks' partial potentials that a call keeps, at most (128 MB).
+constexpr int64_t kGradMaxParts = (int64_t)1 << 24;
 
 // J = 1/2 sum D_pq (pq|rs) D_rs, dJ/dAtomCoords and (optionally) the Coulomb
 // matrix, by the Hermite-vector scheme of grad_engine.cuh.  `dev` says whether
@@ -1832,6 +1834,34 @@ static void coulomb_grad_impl(const gci_basis* basis, double omega, const double
             run[L] += P.h[sp].npp;
         }
     }
+    // ket primitive pairs per warp: 512, which leaves the warp's final sum over its lanes below a
+    // tenth of its work, less where that gives fewer than 16 warps an SM
+    int64_t chunk[NL][NL] = {}, nchunk[NL][NL] = {};
+    GradDotsArgs dp{};
+    int64_t nparts = 0;
+    for (int L1 = 0; L1 < NL; ++L1) {
+        dp.beg[L1] = lbeg[L1];
+        dp.vec_off[L1] = vec_off[L1];
+        dp.pot_off[L1] = pot_off[L1];
+        dp.part_off[L1] = nparts;
+        dp.len[L1] = (int64_t)ln[L1] * grad_hb(L1);
+        for (int L2 = 0; L2 < NL; ++L2) {
+            g_grad_work[L1][L2] = (double)ln[L1] * (double)ln[L2];
+            if (ln[L1] == 0 || ln[L2] == 0) continue;
+            int64_t& c = chunk[L1][L2];
+            c = 512;
+            while (c > 64 && ln[L1] * ((ln[L2] + c - 1) / c) < 148 * 16) c /= 2;
+            nchunk[L1][L2] = (ln[L2] + c - 1) / c;
+            dp.slots[L1] += (int)nchunk[L1][L2];
+        }
+        nparts += dp.slots[L1] * dp.len[L1];
+    }
+    // the classes of a bra level share its potentials and run on different streams: every chunk leaves
+    // its own part, summed in a fixed order, while the parts fit 128 MB (among them every molecule with
+    // at most 512 primitive pairs a level, 75 MB at most; 42 AOs 5 MB), so that equal calls give
+    // equal bits; above it (some 20,000 primitive pairs) the parts' memory would grow with the
+    // square of the molecule, and the chunks are added atomically in whatever order they finish
+    const bool parts = nparts <= kGradMaxParts;
     DVec<int64_t> d_gbase, d_voff, d_hkoff, d_potoff;
     DVec<int> d_lbeg, d_ln, d_ppair;
     DVec<double> mP, mX, mY, mZ, vecs, hk, V, dots, Dd, Jd;
@@ -1846,7 +1876,7 @@ static void coulomb_grad_impl(const gci_basis* basis, double omega, const double
     d_ppair.alloc(n1);
     vecs.alloc((size_t)std::max<int64_t>(nvec, 1));
     hk.alloc((size_t)std::max<int64_t>(nhk, 1));
-    V.alloc((size_t)std::max<int64_t>(npot, 1));
+    V.alloc((size_t)std::max<int64_t>(npot + (parts ? nparts : 0), 1));   // the potentials, then the parts
     dots.alloc(n1 * kGradVec);
     const double* Dp = D;
     if (!dev) {
@@ -1858,33 +1888,35 @@ static void coulomb_grad_impl(const gci_basis* basis, double omega, const double
     CU(grad_pair_vectors_launch(P.d.p, (int)P.n, d_gbase.p, d_lbeg.p, d_ln.p, d_voff.p, d_hkoff.p, db.xyz.p, db.poff.p,
                                 db.exps.p, db.coefs.p, P.plist.p, db.tmat.p, db.toff.p, db.nfunc.p, db.loc.p, Dp, ldd,
                                 mP.p, mX.p, mY.p, mZ.p, vecs.p, hk.p, d_ppair.p, C.stream));
-    CU(cudaMemsetAsync(V.p, 0, sizeof(double) * V.n, C.stream));
-    // the classes only share the potentials, which they add to atomically: spread over the
-    // auxiliary streams, so that the short ones of a small molecule overlap
+    if (!parts) CU(cudaMemsetAsync(V.p, 0, sizeof(double) * npot, C.stream));
     fork_streams(C);
     int li = 0;
-    for (int L1 = 0; L1 < NL; ++L1)
+    for (int L1 = 0; L1 < NL; ++L1) {
+        int64_t slot = 0;
         for (int L2 = 0; L2 < NL; ++L2) {
-            g_grad_work[L1][L2] = (double)ln[L1] * (double)ln[L2];
-            if (ln[L1] == 0 || ln[L2] == 0) continue;
+            if (nchunk[L1][L2] == 0) continue;
             GradPotArgs a{};
             a.mP = mP.p; a.mX = mX.p; a.mY = mY.p; a.mZ = mZ.p;
             a.bra_beg = lbeg[L1]; a.nbra = ln[L1];
             a.ket_beg = lbeg[L2]; a.nket = ln[L2];
             a.hk = hk.p + hk_off[L2];
             a.V = V.p + pot_off[L1];
-            // ket primitive pairs per warp: 512, which leaves the warp's final sum over its lanes
-            // below a tenth of its work, less where that gives fewer than 16 warps an SM
-            a.chunk = 512;
-            while (a.chunk > 64 && a.nbra * ((a.nket + a.chunk - 1) / a.chunk) < 148 * 16) a.chunk /= 2;
-            a.nchunk = (a.nket + a.chunk - 1) / a.chunk;
+            a.part = parts ? V.p + npot + dp.part_off[L1] + slot * dp.len[L1] : nullptr;
+            slot += nchunk[L1][L2];
+            a.chunk = chunk[L1][L2];
+            a.nchunk = nchunk[L1][L2];
             a.kappa = H.kappa;
             a.boys = g_ctx.boys.p;
             CU(grad_potential_launch(L1, L2, a, C.aux[li++ % kAuxStreams]));
         }
+    }
     join_streams(C);
-    for (int L = 0; L < NL; ++L)
-        CU(grad_dots_launch(lbeg[L], ln[L], grad_hb(L), vecs.p + vec_off[L], V.p + pot_off[L], dots.p, C.stream));
+    dp.n = ntot;
+    dp.vecs = vecs.p;
+    dp.V = V.p;
+    dp.part = parts ? V.p + npot : nullptr;
+    dp.out = dots.p;
+    CU(grad_dots_launch(dp, C.stream));
     if (jmat) {
         double* Jp = jmat;
         if (!dev) {
@@ -1901,7 +1933,7 @@ static void coulomb_grad_impl(const gci_basis* basis, double omega, const double
         CU(cudaMemcpyAsync(hd.data(), dots.p, sizeof(double) * (size_t)ntot * kGradVec, cudaMemcpyDeviceToHost,
                            C.stream));
     CU(cudaStreamSynchronize(C.stream));
-    // fixed-order host reduction: deterministic energy and gradient
+    // summed in a fixed order: no bits of its own beside those of the potentials
     double e = 0.0;
     std::vector<double> g((size_t)3 * basis->natoms, 0.0);
     for (int64_t i = 0; i < ntot; ++i) {

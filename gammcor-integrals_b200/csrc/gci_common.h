@@ -238,11 +238,26 @@ struct GradPotArgs {
     int64_t bra_beg, nbra;   // bra primitive pairs of level L1: global indices bra_beg ..
     int64_t ket_beg, nket;   // ket primitive pairs of level L2
     const double* hk;        // ket vectors of level L2, transposed: hk[tau * nket + k], sign (-1)^|tau| applied
-    double* V;               // potentials of level L1: V[i * grad_hb(L1) + t], accumulated atomically
+    double* V;               // potentials of level L1: V[i * grad_hb(L1) + t], accumulated atomically, or
+    double* part;            // (not null) the chunks' parts: part[(c * nbra + i) * grad_hb(L1) + t], stored
     int64_t chunk;           // ket primitive pairs per warp
     int64_t nchunk;          // chunks per bra primitive pair
     double kappa;
     const double* boys;
+};
+
+// Dot products of all primitive pairs (k_grad_dots), those of level L from beg[L] on.
+struct GradDotsArgs {
+    int64_t n;                          // primitive pairs
+    const double* vecs;                 // level L from vec_off[L]: [pair][kGradVec][grad_hb(L)]
+    double* V;                          // level L from pot_off[L]: [pair][grad_hb(L)]
+    // chunks' parts of the potentials to be summed into V (nullptr: V is complete); level L: slots[L]
+    // parts of len[L] entries each, from part_off[L]
+    const double* part;
+    double* out;                        // out[g * kGradVec + c]
+    int64_t beg[kGradMaxL + 1], vec_off[kGradMaxL + 1], pot_off[kGradMaxL + 1], part_off[kGradMaxL + 1],
+        len[kGradMaxL + 1];
+    int slots[kGradMaxL + 1];
 };
 
 } // namespace gci

@@ -98,8 +98,7 @@ cudaError_t grad_pair_vectors_launch(const ShellPairDev* pairs, int npairs, cons
                                      double* mX, double* mY, double* mZ, double* vecs, double* hk, int* ppair,
                                      cudaStream_t st);
 cudaError_t grad_potential_launch(int L1, int L2, const GradPotArgs& a, cudaStream_t st);
-cudaError_t grad_dots_launch(int64_t beg, int64_t n, int HB, const double* vecs, const double* V, double* out,
-                             cudaStream_t st);
+cudaError_t grad_dots_launch(const GradDotsArgs& a, cudaStream_t st);
 cudaError_t grad_coulomb_matrix_launch(const ShellPairDev* pairs, int npairs, const int64_t* gbase,
                                        const int* level_beg, const int64_t* pot_off, const double* V, const double* pp,
                                        const double* tmat, const int* toff, const int* nfunc, const int* loc,

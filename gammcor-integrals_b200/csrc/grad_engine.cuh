@@ -65,7 +65,8 @@ __device__ __forceinline__ double& rget(RLevels<0, N>& R)
 // One warp per (bra primitive pair, chunk of ket primitive pairs); each lane
 // evaluates whole primitive quartets (Boys values, the R_tuv recursion in
 // place, the ket contraction) and accumulates the potential V(t) in
-// registers; the warp's sum is added to V once per chunk.
+// registers; the warp's sum is added to V once per chunk, or stored as the
+// chunk's part.
 template <int L1, int L2>
 __global__ void __launch_bounds__(128) k_grad_potential(const GradPotArgs a)
 {
@@ -135,13 +136,23 @@ __global__ void __launch_bounds__(128) k_grad_potential(const GradPotArgs a)
             });
         });
     }
-    double* Vi = a.V + i * HB;
+    double* Vi = a.part ? a.part + (c * a.nbra + i) * HB : a.V + i * HB;
+    // lane h % 32 keeps entry h, so that rows of 32 are written at once (one write an entry: 42 AOs
+    // 0.91 -> 0.85 ms, 280 AOs 33.8 -> 32.2 ms)
 #pragma unroll
-    for (int h = 0; h < HB; ++h) {
-        double s = Vacc[h];
+    for (int h0 = 0; h0 < HB; h0 += 32) {
+        double mine = 0.0;
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (lane == (h & 31)) atomicAdd(Vi + h, s);
+        for (int h = h0; h < h0 + 32 && h < HB; ++h) {
+            double s = Vacc[h];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            if (lane == h - h0) mine = s;
+        }
+        if (h0 + lane < HB) {
+            if (a.part) Vi[h0 + lane] = mine;
+            else atomicAdd(Vi + h0 + lane, mine);
+        }
     }
 }
 

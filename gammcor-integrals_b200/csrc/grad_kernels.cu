@@ -169,26 +169,45 @@ __global__ void k_grad_pair_vectors(const ShellPairDev* __restrict__ pairs, int 
 
 // One warp per primitive pair: the seven dot products of its vectors with its
 // potential, out[g * 7 + c] (c = 0: h.V, 1..3: gA.V, 4..6: gB.V); the lanes read
-// consecutive entries (one read of the vectors: bound by HBM).
-__global__ void k_grad_dots(int64_t beg, int64_t n, int HB, const double* __restrict__ vecs,
-                            const double* __restrict__ V, double* __restrict__ out)
+// consecutive entries (one read of the vectors: bound by HBM).  Where the chunks
+// left parts of the potential, each lane first adds up those of its entries, in
+// their order: a call's bits then do not depend on the order in which the classes
+// ran.  All levels in one launch: at 42 AOs (up to 26 parts an entry) the reads'
+// latency, sixteen parts in flight, and the launch itself are what it costs.
+__global__ void k_grad_dots(const GradDotsArgs a)
 {
     const int lane = threadIdx.x & 31;
     const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
-    for (int64_t i = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); i < n; i += warps) {
-        const double* vg = vecs + i * (int64_t)(kGradVec * HB);
-        const double* vi = V + i * (int64_t)HB;
+    for (int64_t g = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); g < a.n; g += warps) {
+        int L = 0;
+        while (L < kGradMaxL && g >= a.beg[L + 1]) ++L;
+        const int HB = grad_hb(L);
+        const int64_t i = g - a.beg[L];
+        const double* vg = a.vecs + a.vec_off[L] + i * (int64_t)(kGradVec * HB);
+        double* vi = a.V + a.pot_off[L] + i * (int64_t)HB;
         double s[kGradVec] = {};
         for (int h = lane; h < HB; h += 32) {
-            const double v = vi[h];
+            double w[kGradVec], v = 0.0;
 #pragma unroll
-            for (int c = 0; c < kGradVec; ++c) s[c] = fma(vg[c * HB + h], v, s[c]);
+            for (int c = 0; c < kGradVec; ++c) w[c] = __ldg(vg + c * HB + h);
+            if (a.part) {
+                const double* p = a.part + a.part_off[L] + i * (int64_t)HB + h;
+                const int64_t len = a.len[L];
+                const int slots = a.slots[L];
+#pragma unroll 16
+                for (int q = 0; q < slots; ++q) v += __ldg(p + q * len);
+                vi[h] = v;
+            } else {
+                v = vi[h];
+            }
+#pragma unroll
+            for (int c = 0; c < kGradVec; ++c) s[c] = fma(w[c], v, s[c]);
         }
 #pragma unroll
         for (int c = 0; c < kGradVec; ++c) {
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) s[c] += __shfl_xor_sync(0xffffffffu, s[c], o);
-            if (lane == c) out[(beg + i) * kGradVec + c] = s[c];
+            if (lane == c) a.out[g * kGradVec + c] = s[c];
         }
     }
 }
@@ -308,13 +327,12 @@ cudaError_t grad_potential_launch(int L1, int L2, const GradPotArgs& a, cudaStre
     return cudaGetLastError();
 }
 
-cudaError_t grad_dots_launch(int64_t beg, int64_t n, int HB, const double* vecs, const double* V, double* out,
-                             cudaStream_t st)
+cudaError_t grad_dots_launch(const GradDotsArgs& a, cudaStream_t st)
 {
-    if (n <= 0) return cudaSuccess;
-    int64_t blocks = (n + 3) / 4;
+    if (a.n <= 0) return cudaSuccess;
+    int64_t blocks = (a.n + 3) / 4;
     if (blocks > 148 * 16) blocks = 148 * 16;
-    k_grad_dots<<<(unsigned)blocks, 128, 0, st>>>(beg, n, HB, vecs, V, out);
+    k_grad_dots<<<(unsigned)blocks, 128, 0, st>>>(a);
     count_launch();
     return cudaGetLastError();
 }

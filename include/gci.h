@@ -260,7 +260,11 @@ int gci_autotune_eri(const gci_basis *basis, int max_pairs, double *seconds);
  *   energy  J (may be NULL)
  *   grad    dJ/dAtomCoords, 3 x NAtoms column-major (may be NULL)
  *   jmat    Coulomb matrix J_pq = sum_rs (pq|rs) D_rs = dJ/dD_pq, ldj x NAO (may be NULL).
- * omega <= 0: full-range Coulomb operator. */
+ * omega <= 0: full-range Coulomb operator.
+ * Equal calls give equal bits while the partial potentials fit 128 MB (always where no Hermite level
+ * lA+lB has more than 512 primitive pairs; about 20,000 primitive pairs in all at s, p, d shells);
+ * for larger molecules the potentials are added atomically, in an order that changes from call to
+ * call, and the last digits with it. */
 int gci_coulomb_grad(const gci_basis *basis, double omega, const double *D, int64_t ldd, double *energy,
                      double *grad, double *jmat, int64_t ldj);
 

@@ -7,11 +7,13 @@ torch.autograd.Function.
 
 Tolerances: energy 1e-11 relative; gradient and Coulomb matrix 1e-9 of their
 largest element (FP64 throughout, different summation order); finite
-differences (h = 1e-4 bohr) 1e-6 absolute.
+differences (h = 1e-4 bohr) 1e-6 absolute; repeated calls on one molecule
+equal bits.
 """
 import numpy as np
 import pytest
 
+from gammcor_integrals_b200 import basis as gbasis
 from gammcor_integrals_b200 import coulomb_grad as cgr
 from gammcor_integrals_b200 import molecules
 from oracle import oracle as O
@@ -90,3 +92,20 @@ def test_autograd_function(gpu_lib):
     assert abs(J.item() - e) <= 1e-12 * abs(e)
     np.testing.assert_allclose(coords.grad.cpu().numpy(), 2.5 * g, rtol=0, atol=1e-12 * np.max(np.abs(g)))
     np.testing.assert_allclose(Dt.grad.cpu().numpy(), 2.5 * jm, rtol=0, atol=1e-12 * np.max(np.abs(jm)))
+
+
+@pytest.mark.parametrize("recipe,natoms,nprim", [
+    ((0, 0, 0, 1, 1, 2), 3, (3, 3)),     # small configuration: ket lists in chunks of 64
+    ((0, 1, 2), 4, (9, 9)),              # more than 512 primitive pairs a level
+    ((0, 1, 2, 3), 2, (4, 4)),           # every Hermite level up to 6
+])
+def test_equal_calls_give_equal_bits(gpu_lib, recipe, natoms, nprim):
+    """The classes of a bra level run side by side and share its potentials: their parts are summed
+    in a fixed order."""
+    tb = gbasis.from_molecule(molecules.random_molecule(51, natoms, 5.0, recipe, nprim, (0.1, 50.0)))
+    D = _density(tb.NAO, 51)
+    e, g, jm = cgr.coulomb_energy_grad(tb, D, want_jmat=True)
+    for _ in range(12):
+        e2, g2, jm2 = cgr.coulomb_energy_grad(tb, D, want_jmat=True)
+        assert e2 == e
+        assert np.array_equal(g2, g) and np.array_equal(jm2, jm)
