@@ -11,6 +11,7 @@
 #include "gci_common.h"
 #include "gci_runtime.h"
 #include "host_math.h"
+#include "stream_fork.h"
 #include <algorithm>
 #include <atomic>
 #include <chrono>
@@ -559,21 +560,8 @@ static void hm_ensure_rows(Handle& H, const std::vector<int>& ids)
     for (int64_t id = 0; id < P.n; ++id) H.hm_rowoff_h[id] = want[id] ? off[id] : -1;
 }
 
-// Auxiliary streams of the context, forked from its stream / joined back.  Threads that share a
-// context may interleave: a wait then takes the other thread's later record on the same stream.
-static void fork_streams(Context& C)
-{
-    CU(cudaEventRecord(C.ev_fork, C.stream));
-    for (int q = 0; q < kAuxStreams; ++q) CU(cudaStreamWaitEvent(C.aux[q], C.ev_fork, 0));
-}
-
-static void join_streams(Context& C)
-{
-    for (int q = 0; q < kAuxStreams; ++q) {
-        CU(cudaEventRecord(C.ev_join[q], C.aux[q]));
-        CU(cudaStreamWaitEvent(C.stream, C.ev_join[q], 0));
-    }
-}
+// The auxiliary streams of the context, to be forked from its stream.
+static StreamFork aux_fork(Context& C) { return StreamFork(C.stream, C.aux, kAuxStreams, C.ev_fork, C.ev_join); }
 
 // Column chunks of a Hermite-matrix stage, one set per chunk width in use: rows of level L1
 // take chunks of at most 8 hm_max_nt(L1) columns; within a set, grouped by (column type, tiles).
@@ -737,7 +725,8 @@ static void run_eri_hm(Handle& H, const std::vector<int>& gb, const std::vector<
     if (narrive > 0) CU(cudaMemsetAsync(H.hm_arrive.p, 0, sizeof(int) * narrive, C.stream));
     H.hm_part.ensure((size_t)std::max<int64_t>(part_max * kAuxStreams, 1));
     // the class launches are independent (disjoint outputs): fork them over the auxiliary streams
-    fork_streams(C);
+    StreamFork fork = aux_fork(C);
+    CU(fork.begin());
     const bool prof = g_hm_profile.load() != 0;
     std::vector<std::pair<double*, std::pair<cudaEvent_t, cudaEvent_t>>> timed;
     int64_t li = 0;
@@ -798,7 +787,7 @@ static void run_eri_hm(Handle& H, const std::vector<int>& gb, const std::vector<
                 ++li;
             }
     }
-    join_streams(C);
+    CU(fork.join());
     for (auto& t : timed) {
         float ms = 0.f;
         CU(cudaEventSynchronize(t.second.second));
@@ -877,7 +866,8 @@ static void run_eri(Handle& H, const std::vector<int>& bra, const std::vector<in
     // the diagonal's launches, one a pair type, are each as long as their longest quartet, which one
     // team of lanes evaluates: side by side on the auxiliary streams, the largest types first
     // (60 AOs with f shells 54 -> 26 ms, 360 AOs 113 -> 52 ms, 140 AOs without 2.4 -> 2.0 ms)
-    if (mode == kModeDiagonal) fork_streams(C);
+    StreamFork fork = aux_fork(C);
+    if (mode == kModeDiagonal) CU(fork.begin());
     for (int t = 0; t < kNumPairTypes; ++t) {
         const int tb = kNumPairTypes - 1 - t;
         const int64_t nb = sb[tb + 1] - sb[tb];
@@ -945,7 +935,7 @@ static void run_eri(Handle& H, const std::vector<int>& bra, const std::vector<in
             if (!hm) CU(eri_launch(std::max(tb, tk), std::min(tb, tk), a, C.stream));
         }
     }
-    if (mode == kModeDiagonal) join_streams(C);
+    CU(fork.join());
     if (hm) run_eri_hm(H, gb, sb, gk, sk, mode, rows, cols, out, ldo, jcount, sym);
     if (sym) {
         H.hm_rank.upload(hm_ranks(P, bra, rows->off.data(), rows->map.data(), sym_n), C.stream);
@@ -1889,7 +1879,8 @@ static void coulomb_grad_impl(const gci_basis* basis, double omega, const double
                                 db.exps.p, db.coefs.p, P.plist.p, db.tmat.p, db.toff.p, db.nfunc.p, db.loc.p, Dp, ldd,
                                 mP.p, mX.p, mY.p, mZ.p, vecs.p, hk.p, d_ppair.p, C.stream));
     if (!parts) CU(cudaMemsetAsync(V.p, 0, sizeof(double) * npot, C.stream));
-    fork_streams(C);
+    StreamFork fork = aux_fork(C);   // after the buffers: joined before they are freed
+    CU(fork.begin());
     int li = 0;
     for (int L1 = 0; L1 < NL; ++L1) {
         int64_t slot = 0;
@@ -1910,7 +1901,7 @@ static void coulomb_grad_impl(const gci_basis* basis, double omega, const double
             CU(grad_potential_launch(L1, L2, a, C.aux[li++ % kAuxStreams]));
         }
     }
-    join_streams(C);
+    CU(fork.join());
     dp.n = ntot;
     dp.vecs = vecs.p;
     dp.V = V.p;
