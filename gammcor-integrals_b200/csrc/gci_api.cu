@@ -409,8 +409,7 @@ struct Handle {
     DVec<int> hm_colfun, hm_colout, hm_chunkids;
     DVec<double> hm_colvec;
     DVec<unsigned long long> hm_counters;
-    DVec<int> hm_rank, hm_arrive;
-    DVec<double> hm_part;
+    DVec<int> hm_rank;
     double hm_flops = 0.0;
     // per Hermite-matrix class (L1, L2, column tiles): launches, device seconds
     // (profiling mode only) and DMMA flops issued
@@ -695,7 +694,8 @@ static void run_eri_hm(Handle& H, const std::vector<int>& gb, const std::vector<
     H.hm_counters.ensure((size_t)nlaunch);
     CU(cudaMemsetAsync(H.hm_counters.p, 0, sizeof(unsigned long long) * nlaunch, C.stream));
     // parts of the launches with few tasks: scratch per stream (launches of one stream follow one
-    // another), arrival counters per launch
+    // another), arrival counters per launch; up to 25 MB a stream, so it lives within the stage only
+    // and does not stay with the decompositions that a program keeps
     std::vector<int> split(nlaunch, 1);
     std::vector<int64_t> arrive_off(nlaunch, 0);
     int64_t narrive = 0, part_max = 0;
@@ -721,9 +721,13 @@ static void run_eri_hm(Handle& H, const std::vector<int>& gb, const std::vector<
                 }
         }
     }
-    H.hm_arrive.ensure((size_t)std::max<int64_t>(narrive, 1));
-    if (narrive > 0) CU(cudaMemsetAsync(H.hm_arrive.p, 0, sizeof(int) * narrive, C.stream));
-    H.hm_part.ensure((size_t)std::max<int64_t>(part_max * kAuxStreams, 1));
+    DVec<int> arrive;
+    DVec<double> part;
+    if (narrive > 0) {
+        arrive.alloc((size_t)narrive);
+        part.alloc((size_t)(part_max * kAuxStreams));
+        CU(cudaMemsetAsync(arrive.p, 0, sizeof(int) * narrive, C.stream));
+    }
     // the class launches are independent (disjoint outputs): fork them over the auxiliary streams
     StreamFork fork = aux_fork(C);
     CU(fork.begin());
@@ -771,8 +775,8 @@ static void run_eri_hm(Handle& H, const std::vector<int>& gb, const std::vector<
                 a.counter = H.hm_counters.p + li;
                 a.upper = sym && tk == tb ? 1 : 0;
                 a.split = split[li];
-                a.arrive = H.hm_arrive.p + arrive_off[li];
-                a.part = H.hm_part.p + part_max * (li % kAuxStreams);
+                a.arrive = arrive.p + arrive_off[li];
+                a.part = part.p + part_max * (li % kAuxStreams);
                 if (prof) {
                     cudaEvent_t e0, e1;
                     CU(cudaEventCreate(&e0));

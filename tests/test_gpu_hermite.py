@@ -8,6 +8,9 @@ thousand terms no larger than the largest integral's, in different orders:
 1e-12 of the largest integral (the bound of the ERI parity tests).
 """
 import ctypes as C
+import subprocess
+import sys
+from pathlib import Path
 
 import numpy as np
 import pytest
@@ -74,3 +77,25 @@ def test_noalloc_on_both_sides_of_its_scratch(gpu_lib, nprim):
     got, ref = out.cpu().numpy().T, _eri_pairs(gpu_lib, tb, 0.3, True)
     assert np.max(np.abs(got[:npq] - ref)) <= 1e-12 * np.max(np.abs(ref))
     assert np.all(got[npq:] == 0.0)
+
+
+KEPT = """
+import gammcor_pkg; gammcor_pkg.load()
+import torch
+from gammcor_integrals_b200 import basis, molecules, cholesky_gammcor as cg
+tb = basis.from_molecule(molecules.random_molecule(61, 2, 5.9, molecules.RECIPE_C2, (3, 6), (0.05, 5e3)))
+kept, free = [], []
+for i in range(12):
+    kept.append(cg.chol_gammcor_Rkpq(tb, 2, None, materialize=False, copy_to_host=False))
+    free.append(torch.cuda.mem_get_info()[0])
+print((free[1] - free[11]) / 10 / 2**20)
+"""
+
+
+def test_decompositions_do_not_keep_the_parts(gpu_lib):
+    """Device memory a kept decomposition of 60 AOs with f shells adds, in MB, in a process of its own
+    (the library's pool grows in steps of 32 MB): 45 to 48 with its inverse, Hermite vectors and column
+    data; the parts of four streams would double it (96)."""
+    root = Path(__file__).resolve().parent.parent
+    out = subprocess.run([sys.executable, "-c", KEPT], cwd=root, check=True, capture_output=True, text=True, timeout=300)
+    assert float(out.stdout.split()[-1]) < 72.0
