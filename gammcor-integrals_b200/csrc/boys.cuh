@@ -5,7 +5,7 @@
 // (cheb_approx_5, chebinterp.f90:122-149), then downward recursion
 // F_{k-1} = (2x F_k + e^{-x}) / (2k-1); x >= 25 -> F_0 = sqrt(pi/x)/2 and
 // upward recursion.  The coefficient table is built on the host
-// (boys_table.cpp) and read through the read-only data path.
+// (host_math.cpp) and read through the read-only data path.
 #pragma once
 #include "gci_common.h"
 
@@ -15,7 +15,10 @@ namespace gci {
 // alpha = PQ / (P + Q + kappa PQ) and 2 pi^{5/2} / (PQ sqrt(P + Q + kappa PQ)), both from
 // r = 1 / (PQ sqrt(..)): alpha = (PQ)^3 r^2.  One reciprocal square root where the quotients and
 // the root as written take three times the FP64 instructions (with the one in boys_fm: Coulomb
-// gradient of 280 AOs 38.3 -> 32.6 ms, which this pipe bounds).
+// gradient of 280 AOs 38.3 -> 32.6 ms, which this pipe bounds).  PQ PQ (P + Q + kappa PQ) has to
+// stay a finite number: exponent sums below 1e60.  The class kernels keep the quotients, because the
+// order of tied pivots follows the last bits of the diagonal they evaluate (arguments of boys_fm from
+// kBoysXAsym on changed bits there with its reciprocal root).
 __device__ __forceinline__ void quartet_factors(double P, double Q, double kappa, double& alpha, double& pref)
 {
     const double PQ = P * Q;
@@ -62,38 +65,6 @@ __device__ __forceinline__ void boys_fm(double x, const double* __restrict__ tab
                 f = beta * (static_cast<double>(2 * l - 1) * f - expmx);
                 F[l] = f;
             }
-        }
-    }
-}
-
-// Runtime-order variant used by the Boys self-test entry point.
-__device__ __forceinline__ void boys_fm_rt(int m, double x, const double* __restrict__ table, double* F)
-{
-    if (x < kBoysXAsym) {
-        const int k = static_cast<int>(x * (1.0 / kBoysDelta));
-        const int kk = k < kBoysNInt ? k : kBoysNInt - 1;
-        const double* c = table + (static_cast<size_t>(m) * kBoysNInt + kk) * 5;
-        const double ab_sum = static_cast<double>(2 * kk + 1) * kBoysDelta;
-        const double y = (2.0 * x - ab_sum) * (1.0 / kBoysDelta);
-        const double twoy = 2.0 * y;
-        const double d5 = c[4];
-        const double d4 = twoy * d5 + c[3];
-        const double d3 = twoy * d4 - d5 + c[2];
-        const double d2 = twoy * d3 - d4 + c[1];
-        double f = y * d2 - d3 + 0.5 * c[0];
-        F[m] = f;
-        const double expmx = exp(-x), twox = 2.0 * x;
-        for (int l = m; l >= 1; --l) {
-            f = (twox * f + expmx) / static_cast<double>(2 * l - 1);
-            F[l - 1] = f;
-        }
-    } else {
-        double f = 0.5 * sqrt(kPi / x);
-        F[0] = f;
-        const double expmx = exp(-x), beta = 1.0 / (2.0 * x);
-        for (int l = 1; l <= m; ++l) {
-            f = beta * (static_cast<double>(2 * l - 1) * f - expmx);
-            F[l] = f;
         }
     }
 }

@@ -112,14 +112,23 @@ __global__ void k_pair_records(const ShellPairDev* __restrict__ pairs, int npair
     }
 }
 
-__global__ void k_boys_eval(int m, int64_t n, const double* __restrict__ x, const double* __restrict__ table,
+// boys_fm as the integral kernels call it, one instantiation per order (the self-test's kernel).
+template <int M>
+__global__ void k_boys_eval(int64_t n, const double* __restrict__ x, const double* __restrict__ table,
                             double* __restrict__ out)
 {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        double F[kBoysMaxM + 1];
-        boys_fm_rt(m, x[i], table, F);
-        for (int k = 0; k <= m; ++k) out[i * (m + 1) + k] = F[k];
+        double F[M + 1];
+        boys_fm<M>(x[i], table, F);
+        for (int k = 0; k <= M; ++k) out[i * (M + 1) + k] = F[k];
     }
+}
+
+template <int M = 0>
+static void boys_eval(int m, unsigned blocks, int64_t n, const double* x, const double* table, double* out, cudaStream_t st)
+{
+    if (m == M) k_boys_eval<M><<<blocks, 256, 0, st>>>(n, x, table, out);
+    else if constexpr (M < kBoysMaxM) boys_eval<M + 1>(m, blocks, n, x, table, out, st);
 }
 
 static LaunchFn g_launch[kNumPairTypes][kNumPairTypes];                   // team kernels (bra types up to (d,d))
@@ -198,7 +207,8 @@ cudaError_t boys_eval_launch(int m, int64_t n, const double* x, const double* ta
     if (n <= 0) return cudaSuccess;
     int64_t blocks = (n + 255) / 256;
     if (blocks > 148 * 16) blocks = 148 * 16;
-    k_boys_eval<<<(unsigned)blocks, 256, 0, st>>>(m, n, x, table, out);
+    if (m < 0 || m > kBoysMaxM) return cudaErrorInvalidValue;
+    boys_eval(m, (unsigned)blocks, n, x, table, out, st);
     count_launch();
     return cudaGetLastError();
 }
