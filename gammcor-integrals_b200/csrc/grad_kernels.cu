@@ -172,8 +172,9 @@ __global__ void k_grad_pair_vectors(const ShellPairDev* __restrict__ pairs, int 
 // consecutive entries (one read of the vectors: bound by HBM).  Where the chunks
 // left parts of the potential, each lane first adds up those of its entries, in
 // their order: a call's bits then do not depend on the order in which the classes
-// ran.  All levels in one launch: at 42 AOs (up to 26 parts an entry) the reads'
-// latency, sixteen parts in flight, and the launch itself are what it costs.
+// ran.  All levels in one launch: at 42 AOs (up to 26 parts an entry) 10 us, the
+// latency of the reads (16 us with the vectors read after the parts and eight parts
+// in flight), where a launch a level took 20 on potentials that came summed.
 __global__ void k_grad_dots(const GradDotsArgs a)
 {
     const int lane = threadIdx.x & 31;
