@@ -280,6 +280,8 @@ __global__ void __launch_bounds__(kGradMatThreads) k_grad_coulomb_matrix(const S
         const int64_t l1 = loc[s1], l2 = loc[s2];
         for (int e = threadIdx.x; e < nf1 * nf2; e += blockDim.x) {
             const int ma = e / nf2, mb = e - ma * nf2;
+            // a shell with itself: (ma, mb) and (mb, ma) differ in their last bits, one of them counts
+            if (s1 == s2 && ma < mb) continue;
             double acc = 0.0;
             for (int b = 0; b < nc2; ++b) acc += Jh[ma * nc2 + b] * T2[mb * nc2 + b];
             J[(l1 + ma) + ldj * (l2 + mb)] = acc;
